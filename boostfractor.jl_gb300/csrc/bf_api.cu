@@ -497,7 +497,7 @@ size_t bf_stack_device_bytes(const bf_stack* s) {
              sizeof(RegionGeo) * s->nd;
   if (s->d_surf) b += sizeof(double2) * s->nd * npix;
   if (const Workspace* w = s->ws) {
-    for (const DBuf* d : {&w->freq, &w->reg, &w->phasor, &w->tidx, &w->tregs, &w->tilt, &w->init, &w->state,
+    for (const DBuf* d : {&w->freq, &w->reg, &w->phasor, &w->tab_idx, &w->compact_A, &w->tidx, &w->tregs, &w->tilt, &w->init, &w->state,
                           &w->add, &w->coef, &w->exitacc, &w->steps, &w->tmp, &w->beta, &w->mg, &w->exit_full[0],
                           &w->exit_full[1], &w->direct[0], &w->direct[1]})
       b += dbuf_bytes(*d);
@@ -512,6 +512,44 @@ void bf_stack_trim(bf_stack* s) {
   s->ws = nullptr;
   if (s->tf_cache && s->tf_cache_delete) s->tf_cache_delete(s->tf_cache);
   s->tf_cache = nullptr;
+}
+
+// Transform length of the stack's bounce stages, 0 when only the full-grid
+// path can run them.  The truncated kernel's length where it is shorter than
+// the grid (N = 128 and a 38-pixel box: 80, 0.39 of the points in the column
+// pass) or the grid has no transform of its own (not a power of two, above
+// 256); it takes one quadrant of phasors, so kX and kY antisymmetric.
+static int fused_length(const bf_stack* s, bool fp64) {
+  if (s->nx != s->ny || s->nx < 8) return 0;
+  const int n = s->nx;
+  const int own = bf::fused_supported(n, s->nbx, s->nby, fp64) && (n & (n - 1)) == 0 ? n : 0;
+  const int M = s->kx_sym ? bf::compact_length(std::max(s->nbx, s->nby), fp64) : 0;
+  if (M && (!own || M < own) && n <= 1024 && bf::fused_supported(M, s->nbx, s->nby, fp64)) return M;
+  return own;
+}
+
+// Whether the bounce stages run in complex128: always on the FP64 path, and at
+// mixed precision on grids whose own length has no complex64 transform (not a
+// power of two, or above 256).  The full-grid path that such a mixed solve took
+// before sums its line transforms in FP64, at an error of 5e-8 to 3e-6 in
+// beta^2; complex64 stages reached only 5e-8 to 9e-6 there, complex128 ones
+// 1e-15, and are still 30 times faster than the full grid (101 points, one
+// disk, 32 frequencies, 101 bounces: 26 ms against 880).
+static bool stages_fp64(const bf_stack* s, int precision) {
+  return precision == BF_PREC_FP64 || s->nx > 256 || (s->nx & (s->nx - 1)) != 0;
+}
+
+// Whether the fused solve's failure `rc` leaves the full-grid path to try: out
+// of memory on a grid that only the truncated kernel brought to the fused
+// stages (they hold more bytes a frequency than the full grid's fields when
+// the box fills most of the grid).
+static bool retry_full(bf_handle* h, bf_stack* s, bool wide, int rc) {
+  const int n = s->nx;
+  if (rc != BF_ERR_NOMEM || ((n & (n - 1)) == 0 && bf::fused_supported(n, s->nbx, s->nby, wide))) return false;
+  delete s->ws;
+  s->ws = nullptr;
+  h->err.clear();
+  return true;
 }
 
 size_t bf_solve_bytes_estimate(const bf_stack* s, int solver, int nf, int nm, int prop_kind, int precision) {
@@ -541,9 +579,13 @@ size_t bf_solve_bytes_estimate(const bf_stack* s, int solver, int nf, int nm, in
   // split-phase row tiles: at most (SMs = 160 here, an upper bound) step x
   // frequency pairs of two nby x (N + 2) tiles, or every step's when no stage
   // fits the fused kernel's shared memory
-  const bool split_only = bf::fused_split_only(s->nx, s->nbx, s->nby, precision == BF_PREC_FP64);
-  const size_t split = (split_only ? nd * F : 160) * 2 * (size_t)s->nby * (s->nx + 2) * csz;
-  const size_t fused = F * (csz * (slots * plane + nd * npix + nd * plane) + 16 * (2 * plane + 3 * npix)) + split;
+  const bool wide = stages_fp64(s, precision);
+  const size_t fsz = wide ? 16 : 8;
+  const int M = fused_length(s, wide);
+  const bool split_only = M && bf::fused_split_only(M, s->nbx, s->nby, wide);
+  const size_t split = (split_only ? nd * F : 160) * 2 * (size_t)s->nby * (M + 4) * fsz;
+  const size_t table = M && M != s->nx ? (size_t)M * M / 4 : npix;   // a quadrant, at most the grid
+  const size_t fused = F * (fsz * (slots * plane + nd * table + nd * plane) + 16 * (2 * plane + 3 * npix)) + split;
   const size_t full = F * (csz * (slots + 1) * npix + 16 * 3 * npix);
   return std::max(fused, full) + F * 64;
 }
@@ -1002,7 +1044,7 @@ extern "C" int bf_autotune_report(char* out, int cap) {
 extern "C" int bf_test_force_fused_variant(int v) { return g_force_variant.exchange(v); }
 
 template <typename C>
-static int fused_autotune(bf_handle* h, const Workspace& w, const bf::FusedArgs<C>& a, int N, bool fp64,
+static int fused_autotune(bf_handle* h, const Workspace& w, const bf::FusedArgs<C>& a, int grid, int N, bool fp64,
                           cudaStream_t st, int* out) {
   *out = bf::kFusedRule;
   if (g_force_variant.load() >= 0) {
@@ -1030,7 +1072,7 @@ static int fused_autotune(bf_handle* h, const Workspace& w, const bf::FusedArgs<
   cand.erase(cand.begin());   // the rule's choice is one of the explicit variants
   size_t kbest = (size_t)-1, lbest = 0;
   for (size_t k = 0; k < w.stage_len.size(); ++k)
-    if ((N < 64 || !bf::split_stage((int)w.stage_len[k], a.nfreq)) && w.stage_len[k] > lbest) {
+    if ((!bf::split_length(N) || !bf::split_stage((int)w.stage_len[k], a.nfreq)) && w.stage_len[k] > lbest) {
       lbest = w.stage_len[k];
       kbest = k;
     }
@@ -1098,7 +1140,7 @@ static int fused_autotune(bf_handle* h, const Workspace& w, const bf::FusedArgs<
     std::lock_guard<std::mutex> lock(g_tune_mu);
     g_fused_tuned[key] = best;
   }
-  bf_tune_log("fused N=" + std::to_string(N) + " box=" + std::to_string(a.nbx) + "x" + std::to_string(a.nby) +
+  bf_tune_log("fused N=" + std::to_string(grid) + " transform=" + std::to_string(N) + " box=" + std::to_string(a.nbx) + "x" + std::to_string(a.nby) +
               (fp64 ? " c128" : " c64") + " nf=" + std::to_string(a.nfreq) + " -> variant " + std::to_string(best) +
               " (ms per launch of " + std::to_string(lbest) + " steps:" + what + ")");
   *out = best;
@@ -1112,11 +1154,26 @@ static int run_fused(bf_handle* h, bf_stack* s, const std::string& key,
   cudaStream_t st = h->stream();
   if (!s->ws) s->ws = new Workspace();
   Workspace& w = *s->ws;
-  const int N = s->nx;
+  const int n = s->nx, N = fused_length(s, fp64);
   const size_t plane = (size_t)s->nbx * s->nby;
   const size_t npix = (size_t)s->nx * s->ny;
   const size_t csz = sizeof(C);
   const int fold = s->kx_sym ? 1 : 0;
+  // the truncated kernel's transform: its fields carry exp(i alpha (x + y)),
+  // which makes the spectra of an even grid's half-integer wavenumbers and of
+  // the transform's even in each axis (one quadrant); everything between two
+  // propagations is pointwise, so the factor goes in once with the emission
+  // and comes out once at the exits
+  const bool compact = N != n || (n & (n - 1)) != 0;
+  const double alpha = compact ? M_PI * ((n % 2 == 0 ? 1.0 / n : 0.0) - 1.0 / N) : 0.0;
+  auto modulate = [&](std::vector<cd>& boxes) {
+    if (alpha == 0.0) return;
+    for (size_t i = 0; i < boxes.size(); ++i) {
+      const size_t p = i % plane;
+      const double t = alpha * (double)(p / s->nbx + p % s->nbx);
+      boxes[i] *= cd(std::cos(t), std::sin(t));
+    }
+  };
   const int QW = fold ? N / 2 : N;
   const std::string full_key = key + "|v" + std::to_string(s->geo_version) + (fp64 ? "|d" : "|f");
   prof_mark(h, 0);
@@ -1132,7 +1189,11 @@ static int run_fused(bf_handle* h, bf_stack* s, const std::string& key,
     w.nexit = p.nexit;
     w.exit_region = p.exit_region;
     w.exit_coef = p.exit_coef;
-    CKS(upload(h, w.reg, p.tab_region.data(), sizeof(int) * w.ntab));
+    w.tab_region = p.tab_region;
+    if (compact) {
+      const std::vector<double> A = bf::compact_matrix(n, N, std::max(s->nbx, s->nby));
+      CKS(upload(h, w.compact_A, A.data(), sizeof(double) * A.size()));
+    }
     std::vector<int> tidx(w.ntab, -1), tregs;
     for (int t = 0; t < w.ntab; ++t) {
       const int reg = p.tab_region[t];
@@ -1146,26 +1207,24 @@ static int run_fused(bf_handle* h, bf_stack* s, const std::string& key,
     if (w.ntilt) CKS(upload(h, w.tregs, tregs.data(), sizeof(int) * w.ntilt));
     std::vector<cd> init((size_t)p.nslots * plane);
     for (int k = 0; k < p.nslots; ++k) std::copy(p.init[k].begin(), p.init[k].end(), init.begin() + k * plane);
+    modulate(init);
     CKS(upload_cd_as(h, w.init, init));
     w.nadd = (int)p.adds.size();
     if (w.nadd) {
       std::vector<cd> adds(p.adds.size() * plane);
       for (size_t k = 0; k < p.adds.size(); ++k) std::copy(p.adds[k].begin(), p.adds[k].end(), adds.begin() + k * plane);
+      modulate(adds);
       DBuf b_add64;
       CKS(upload_cd_as(h, b_add64, adds));
       CKS(w.add.alloc(h, csz * adds.size()));
       CKL(bf::launch_convert(b_add64.p, true, w.add.p, fp64, adds.size(), st));
       CK(cudaStreamSynchronize(st));
     }
-    std::vector<double2> coefs(4 * p.coefs.size());
-    for (size_t k = 0; k < p.coefs.size(); ++k) {
-      const Coef4& c = p.coefs[k];
-      coefs[4 * k + 0] = make_double2(c.aa.real(), c.aa.imag());
-      coefs[4 * k + 1] = make_double2(c.ab.real(), c.ab.imag());
-      coefs[4 * k + 2] = make_double2(c.ba.real(), c.ba.imag());
-      coefs[4 * k + 3] = make_double2(c.bb.real(), c.bb.imag());
-    }
-    CKS(upload(h, w.coef, coefs.data(), sizeof(double2) * coefs.size()));
+    using R = decltype(C().x);
+    std::vector<C> coefs;
+    for (const Coef4& c : p.coefs)
+      for (const cd& v : {c.aa, c.ab, c.ba, c.bb}) coefs.push_back(bf::mk((R)v.real(), (R)v.imag()));
+    CKS(upload(h, w.coef, coefs.data(), sizeof(C) * coefs.size()));
     std::vector<StepDesc> all;
     w.stage_off.clear();
     w.stage_len.clear();
@@ -1194,9 +1253,26 @@ static int run_fused(bf_handle* h, bf_stack* s, const std::string& key,
   if (new_tables) {
     CKS(w.freq.ensure(h, sizeof(double) * nf));
     CK(cudaMemcpyAsync(w.freq.p, freqs, sizeof(double) * nf, cudaMemcpyHostToDevice, st));
+    // regions of equal thickness and permittivity (the disks of a booster) share a table
+    std::vector<int> regs, idx(w.ntab);
+    for (int t = 0; t < w.ntab; ++t) {
+      const int r = w.tab_region[t];
+      size_t k = 0;
+      while (k < regs.size() && !(s->distance[regs[k]] == s->distance[r] && s->eps[regs[k]] == s->eps[r])) ++k;
+      if (k == regs.size()) regs.push_back(r);
+      idx[t] = (int)k;
+    }
+    CKS(w.reg.ensure(h, sizeof(int) * w.ntab));
+    CK(cudaMemcpyAsync(w.reg.p, regs.data(), sizeof(int) * regs.size(), cudaMemcpyHostToDevice, st));
+    CKS(w.tab_idx.ensure(h, sizeof(int) * w.ntab));
+    CK(cudaMemcpyAsync(w.tab_idx.p, idx.data(), sizeof(int) * w.ntab, cudaMemcpyHostToDevice, st));
     CKS(w.phasor.ensure(h, csz * (size_t)nf * w.ntab * QW * QW));
-    CKL(bf::launch_phasor_table(fp64, w.phasor.p, nf, w.freq.as<double>(), w.ntab, w.reg.as<int>(), s->d_geo, N,
-                                s->dkX, s->dkY, fold, st));
+    if (compact)
+      CKL(bf::launch_compact_table(fp64, w.phasor.p, nf, w.freq.as<double>(), (int)regs.size(), w.ntab,
+                                   w.reg.as<int>(), s->d_geo, n, s->dkX, s->dkY, w.compact_A.as<double>(), N, st));
+    else
+      CKL(bf::launch_phasor_table(fp64, w.phasor.p, nf, w.freq.as<double>(), (int)regs.size(), w.ntab,
+                                  w.reg.as<int>(), s->d_geo, N, s->dkX, s->dkY, fold, st));
     if (w.ntilt) {
       CKS(w.tilt.ensure(h, csz * (size_t)nf * w.ntilt * plane));
       CKL(bf::launch_tilt_table(fp64, w.tilt.p, nf, w.freq.as<double>(), w.ntilt, w.tregs.as<int>(), s->d_geo,
@@ -1216,11 +1292,12 @@ static int run_fused(bf_handle* h, bf_stack* s, const std::string& key,
   a.nfreq = nf; a.nbx = s->nbx; a.nby = s->nby; a.nslots = w.nslots; a.ntab = w.ntab; a.fold = fold;
   a.state = w.state.as<C>();
   a.phasor = w.phasor.as<C>();
+  a.tab_idx = w.tab_idx.as<int>();
   a.tilt = w.ntilt ? w.tilt.as<C>() : nullptr;
   a.tilt_idx = w.tidx.as<int>();
   a.ntilt = w.ntilt;
   a.mask = s->d_mask_box;
-  a.coefs = w.coef.as<double2>();
+  a.coefs = w.coef.as<C>();
   a.exitacc = w.exitacc.as<double2>();
   a.addbuf = w.nadd ? w.add.as<C>() : nullptr;
   a.err = reinterpret_cast<int*>(h->d_scalar + 1);
@@ -1233,7 +1310,7 @@ static int run_fused(bf_handle* h, bf_stack* s, const std::string& key,
     for (size_t len : w.stage_len)
       if (split_only || bf::split_stage((int)len, nf)) split_len = std::max(split_len, len);
     a.mg = nullptr;
-    if (split_len && N >= 64) {
+    if (split_len && bf::split_length(N)) {
       CKS(w.mg.ensure(h, bf::split_tile_bytes(N, s->nby, nf, (int)split_len, fp64)));
       a.mg = w.mg.as<C>();
     }
@@ -1241,7 +1318,7 @@ static int run_fused(bf_handle* h, bf_stack* s, const std::string& key,
   a.variant = bf::kFusedRule;
   {
     int v = bf::kFusedRule;
-    CKS(fused_autotune<C>(h, w, a, N, fp64, st, &v));
+    CKS(fused_autotune<C>(h, w, a, n, N, fp64, st, &v));
     a.variant = v;
   }
   prof_mark(h, 1);
@@ -1264,7 +1341,7 @@ static int run_fused(bf_handle* h, bf_stack* s, const std::string& key,
   std::string gkey = key + (fp64 ? "|d" : "|f");
   {
     const void* ptrs[] = {a.state, a.phasor, a.tilt, a.tilt_idx, a.mask, a.coefs, a.exitacc, a.addbuf,
-                          a.err, w.steps.p, a.mg};
+                          a.err, w.steps.p, a.mg, a.tab_idx};
     const long long ints[] = {nf, a.nbx, a.nby, a.nslots, a.ntab, a.fold, a.ntilt, N, (long long)fp64,
                               (long long)w.stage_off.size(), h->device, a.variant};
     gkey.append(reinterpret_cast<const char*>(ptrs), sizeof(ptrs));
@@ -1320,7 +1397,7 @@ static int run_fused(bf_handle* h, bf_stack* s, const std::string& key,
   for (int k = 0; k < w.nexit; ++k) {
     CKS(w.exit_full[k].ensure(h, sizeof(double2) * nf * npix));
     CKL(bf::launch_embed_box(w.exit_full[k].as<double2>(), w.exitacc.as<double2>() + (size_t)k * nf * plane, nf,
-                             s->nx, s->ny, s->nbx, s->nby, s->bx0, s->by0, st));
+                             s->nx, s->ny, s->nbx, s->nby, s->bx0, s->by0, alpha, st));
     CKS(general_prop(h, s, BF_PROP_3D, true, w.exit_full[k].p, w.tmp.p, nf, w.freq.as<double>(), w.exit_region[k]));
     cd c = w.exit_coef[k];
     CKL(bf::launch_exit_combine(w.exit_full[k].as<double2>(), w.exit_full[k].as<double2>(),
@@ -1803,8 +1880,9 @@ extern "C" int bf_stack_cheerleader(bf_handle* h, bf_stack* s, int nf, const dou
     CK(cudaStreamSynchronize(st));
     return BF_OK;
   }
-  const bool fusable = (prop_kind == BF_PROP_3D || prop_kind == BF_PROP_NOTILTS) && amin == 0.0 &&
-                       s->nx == s->ny && bf::fused_supported(s->nx, s->nbx, s->nby, fp64);
+  const bool wide = stages_fp64(s, precision);
+  bool fusable = (prop_kind == BF_PROP_3D || prop_kind == BF_PROP_NOTILTS) && amin == 0.0 &&
+                 fused_length(s, wide) != 0;
   if (fusable) {
     // NOTILTS: the tilt maps are identity, as if tilts and surfaces were zero
     bf_stack* sp = s;
@@ -1824,7 +1902,7 @@ extern "C" int bf_stack_cheerleader(bf_handle* h, bf_stack* s, int nf, const dou
       plan_cheerleader(sp, nmax, em, p);
     };
     std::vector<const double2*> ex;
-    int rc = fp64 ? run_fused<double2>(h, sp, key, mk, true, nf, freqs, ex)
+    int rc = wide ? run_fused<double2>(h, sp, key, mk, true, nf, freqs, ex)
                   : run_fused<float2>(h, sp, key, mk, false, nf, freqs, ex);
     if (rc == BF_OK) {
       rc = deliver(h, out_right, ex[0], sizeof(double2) * nf * npix, flags);
@@ -1833,9 +1911,11 @@ extern "C" int bf_stack_cheerleader(bf_handle* h, bf_stack* s, int nf, const dou
     }
     if (rc == BF_OK) rc = finish_profile(h);
     if (rc == BF_OK) rc = check_device_error(h);
+    fusable = !retry_full(h, sp, wide, rc);
     if (sp != s) { delete tmp_stack.ws; tmp_stack.ws = nullptr; }
-    if (rc != BF_OK) return rc;
-  } else {
+    if (fusable && rc != BF_OK) return rc;
+  }
+  if (!fusable) {
     int n_done = 0;
     cheer_emission(s, emit, reflect, em);
     DBuf b_freq;
@@ -1867,9 +1947,9 @@ extern "C" int bf_stack_dancer(bf_handle* h, bf_stack* s, int nf, const double* 
     dancer_emission(s, emit, reflect, em);
     CKS(run_1d(h, s, 1, nf, hfreq, amin, nmax, em, per_iter, exits));
   } else {
-    const bool fusable = (prop_kind == BF_PROP_3D || prop_kind == BF_PROP_NOTILTS) && amin == 0.0 &&
-                         !per_iter && s->nx == s->ny &&
-                         bf::fused_supported(s->nx, s->nbx, s->nby, fp64);
+    const bool wide = stages_fp64(s, precision);
+    bool fusable = (prop_kind == BF_PROP_3D || prop_kind == BF_PROP_NOTILTS) && amin == 0.0 &&
+                   !per_iter && fused_length(s, wide) != 0;
     if (fusable) {
       bf_stack* sp = s;
       bf_stack tmp_stack;
@@ -1889,7 +1969,7 @@ extern "C" int bf_stack_dancer(bf_handle* h, bf_stack* s, int nf, const double* 
         plan_dancer(sp, nmax, em, p);
       };
       std::vector<const double2*> ex;
-      int rc = fp64 ? run_fused<double2>(h, sp, key, mk, true, nf, freqs, ex)
+      int rc = wide ? run_fused<double2>(h, sp, key, mk, true, nf, freqs, ex)
                     : run_fused<float2>(h, sp, key, mk, false, nf, freqs, ex);
       if (rc == BF_OK) {
         rc = deliver(h, out, ex[0], sizeof(double2) * nf * npix, flags);
@@ -1897,11 +1977,15 @@ extern "C" int bf_stack_dancer(bf_handle* h, bf_stack* s, int nf, const double* 
         if (rc == BF_OK) rc = finish_profile(h);
         if (rc == BF_OK) rc = check_device_error(h);
       }
+      fusable = !retry_full(h, sp, wide, rc);
       if (sp != s) { delete tmp_stack.ws; tmp_stack.ws = nullptr; }
-      if (rc != BF_OK) return rc;
-      CK(cudaStreamSynchronize(st));
-      return BF_OK;
-    } else {
+      if (fusable) {
+        if (rc != BF_OK) return rc;
+        CK(cudaStreamSynchronize(st));
+        return BF_OK;
+      }
+    }
+    if (!fusable) {
       dancer_emission(s, emit, reflect, em);
       DBuf b_freq;
       CKS(upload(h, b_freq, freqs, sizeof(double) * nf));

@@ -19,11 +19,12 @@
 #include <stdio.h>
 
 #include <algorithm>
+#include <type_traits>
 #include <vector>
 
 #include "bf_common.cuh"
 #include "bf_device.cuh"
-#include "bf_fft.cuh"
+#include "bf_stage.cuh"
 
 namespace bf {
 
@@ -37,49 +38,21 @@ void note_launches(unsigned long long n) { g_launches += n; }
 void unnote_launches(unsigned long long n) { g_launches -= n; }
 #define COUNT_LAUNCH() (++g_launches)
 
-// Round an FP64 complex value to complex64 so that the modulus error is as
-// small as possible: of the float pairs within one ulp of (re, im) take the one
-// whose squared modulus is closest to the FP64 one.  Plain rounding leaves a
-// random modulus error of ~6e-8 per value, and a phasor or twiddle that is
-// applied to the same k-bin on every bounce turns that into a systematic gain
-// or loss that compounds over hundreds of bounces.
-__host__ __device__ inline float2 round_c64_host_device(double re, double im) {
-  const float fr = (float)re, fi = (float)im;
-  const double m2 = re * re + im * im;
-  float best_r = fr, best_i = fi;
-  double best = 1e300;
-  for (int a = -1; a <= 1; ++a)
-    for (int b = -1; b <= 1; ++b) {
-      float cr = a == 0 ? fr : nextafterf(fr, a > 0 ? INFINITY : -INFINITY);
-      float ci = b == 0 ? fi : nextafterf(fi, b > 0 ? INFINITY : -INFINITY);
-      double d = fabs((double)cr * cr + (double)ci * ci - m2);
-      // prefer the plain rounding on ties (keeps exact values exact)
-      if (d < best || (d == best && a == 0 && b == 0)) {
-        best = d;
-        best_r = cr;
-        best_i = ci;
-      }
-    }
-  return make_float2(best_r, best_i);
-}
-
-void init_constant_roots() {
-  static double2 hd[1024];
-  static float2 hf[1024];
-  for (int k = 0; k < 1024; ++k) {
-    // exp(-2 pi i k / 1024); cos/sin evaluated on the first octant and mapped
-    // by symmetry so that the table is exactly symmetric
-    int q = k / 256, r = k % 256;
+void fill_roots(int n, double2* hd, float2* hf) {
+  for (int k = 0; k < n; ++k) {
+    // cos/sin evaluated on the first octant and mapped by symmetry so that
+    // the table is exactly symmetric
+    int q = k / (n / 4), r = k % (n / 4);
     double c, s;
-    int rr = r <= 128 ? r : 256 - r;
-    double a = M_PI * rr / 512.0;
+    int rr = r <= n / 8 ? r : n / 4 - r;
+    double a = 2.0 * M_PI * rr / n;
     double cr = cos(a), sr = sin(a);
-    if (r > 128) { double t = cr; cr = sr; sr = t; }
+    if (r > n / 8) { double t = cr; cr = sr; sr = t; }
     // float copy of the first-octant pair, rounded for the smallest modulus error,
     // then mapped by the same exact symmetry as the FP64 pair
     const float2 o = round_c64_host_device(cr, sr);
     float cf, sf;
-    // angle theta = 2 pi k / 1024 = q*pi/2 + 2 pi r/1024; (cos, sin) of theta
+    // angle theta = 2 pi k / n = q*pi/2 + 2 pi r/n; (cos, sin) of theta
     switch (q) {
       case 0: c = cr; s = sr; cf = o.x; sf = o.y; break;
       case 1: c = -sr; s = cr; cf = -o.y; sf = o.x; break;
@@ -89,8 +62,12 @@ void init_constant_roots() {
     hd[k] = make_double2(c, -s);
     hf[k] = make_float2(cf, -sf);
   }
-  cudaMemcpyToSymbol(c_root1024_d, hd, sizeof(hd));
-  cudaMemcpyToSymbol(c_root1024_f, hf, sizeof(hf));
+}
+
+void init_constant_roots() {
+  upload_roots();
+  init_roots_five_f();
+  init_roots_five_d();
 }
 
 // ---------------------------------------------------------------------------
@@ -140,589 +117,7 @@ __device__ __forceinline__ double2 phase_k0c(double2 k0, double2 s) {
   return dcexp(im, -re);
 }
 
-template <typename C> __device__ __forceinline__ C from_d(double2 v);
-template <> __device__ __forceinline__ float2 from_d<float2>(double2 v) {
-  return make_float2((float)v.x, (float)v.y);
-}
-template <> __device__ __forceinline__ double2 from_d<double2>(double2 v) { return v; }
-// phase factors: modulus-aware rounding to complex64
-template <typename C> __device__ __forceinline__ C from_d_phase(double2 v);
-template <> __device__ __forceinline__ float2 from_d_phase<float2>(double2 v) {
-  return round_c64_host_device(v.x, v.y);
-}
-template <> __device__ __forceinline__ double2 from_d_phase<double2>(double2 v) { return v; }
-template <typename C> __device__ __forceinline__ C czero() { return from_d<C>(make_double2(0.0, 0.0)); }
-
 #define SPEED_OF_LIGHT 299792458.0
-
-// ---------------------------------------------------------------------------
-// Fused box stage kernel
-// ---------------------------------------------------------------------------
-constexpr int kFusedThreads = 256;
-constexpr int kSmemHeader = 128;
-
-template <int N> __host__ __device__ constexpr int fused_pitch() { return N + 2; }
-
-// Kernel-shape options of the fused stage (a bit mask): the inter-pass
-// twiddles from a shared table instead of registers; team exchanges in two
-// halves through half-size scratch; each column task's folded phasor row
-// copied into the team's shared buffer (cp.async) while the team runs the
-// forward transform, instead of loaded from L2 after it.  None changes the
-// arithmetic.
-constexpr int kModeTwShared = 1, kModeHalf = 2, kModeStage = 4;
-
-// Complex elements of one team's shared region: its exchange scratch, then
-// (kModeStage) the N/2-entry phasor row buffer.
-template <int N, int MODE> __host__ __device__ constexpr int team_region() {
-  return Team<N>::template scratch<(MODE & kModeHalf) != 0>() + ((MODE & kModeStage) ? N / 2 : 0);
-}
-
-__device__ __forceinline__ void cp_async16(void* dst_smem, const void* src_global) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((unsigned)__cvta_generic_to_shared(dst_smem)),
-               "l"(src_global)
-               : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_group 0;" ::: "memory"); }
-
-template <typename C, int N>
-struct FusedCtx {
-  using T = Team<N>;
-  static constexpr int G = T::G, RR = T::RR, CC = T::C;
-  static constexpr int P = fused_pitch<N>();
-};
-
-// Phase 1 of one propagation: forward FFT along x of every box row.  Fields
-// are stored pre-masked, so only register slots r < ceil(nbx/G) can hold box
-// pixels.  A slot feeding an exit adds its (masked) input to the FP64 exit
-// accumulator on the way.
-template <typename C, int N, int NZ, int NT, bool HALF = false>
-__device__ __forceinline__ void fused_phase1(const FusedArgs<C>& a, int f, int slot, int exitk, C* M,
-                                             C* scr, const C* tw, int team, int g) {
-  using X = FusedCtx<C, N>;
-  constexpr int G = X::G, RR = X::RR, CC = X::CC, P = X::P;
-  constexpr int NTEAM = NT;
-  const int nbx = a.nbx, nby = a.nby;
-  const C* src = a.state + ((size_t)f * a.nslots + slot) * (size_t)(nby * nbx);
-  double2* acc = exitk >= 0 ? a.exitacc + ((size_t)exitk * a.nfreq + f) * (size_t)(nby * nbx) : nullptr;
-  const int rv = (nbx + G - 1) / G;
-  for (int base = 0; base < nby; base += NTEAM) {
-    const int y = base + team;
-    const bool act = y < nby;
-    if (!__any_sync(0xffffffffu, act)) continue;   // the whole warp is idle
-    const C* row = src + y * nbx;
-    double2* arow = acc ? acc + y * nbx : nullptr;
-    C v[RR];
-#pragma unroll
-    for (int r = 0; r < RR; ++r) {
-      v[r] = czero<C>();
-      if (r < NZ && r < rv) {
-        const int x = g + G * r;
-        if (act && x < nbx) {
-          const C val = row[x];
-          v[r] = val;
-          if (arow) {
-            double2 o = arow[x];
-            double2 d = to_d(val);
-            arow[x] = make_double2(o.x + d.x, o.y + d.y);
-          }
-        }
-      }
-    }
-    X::T::template forward<NZ, HALF>(v, tw, scr, g);
-    if (act) {
-#pragma unroll
-      for (int j = 0; j < CC; ++j)
-#pragma unroll
-        for (int q = 0; q < G; ++q) M[y * P + g * CC + j + RR * q] = v[j * G + q];
-    }
-  }
-  __syncthreads();
-}
-
-// Phase 2: per column kx, forward FFT along y, phasor, inverse FFT along y,
-// in place in M (only the nby box rows are read and written).  STAGE: the
-// column's folded phasor row is copied into the team's buffer behind its
-// scratch (cp.async, issued before the forward transform) and read from there.
-template <typename C, int N, int NZ, int NT, bool HALF = false, bool STAGE = false>
-__device__ __forceinline__ void fused_phase2(const FusedArgs<C>& a, const C* Q, C* M, C* scr,
-                                             const C* tw, int team, int g) {
-  using X = FusedCtx<C, N>;
-  constexpr int G = X::G, RR = X::RR, CC = X::CC, P = X::P;
-  constexpr int NTEAM = NT;
-  const int nby = a.nby;
-  const int QW = a.fold ? N / 2 : N;
-  const int rv = (nby + G - 1) / G;
-  C* qb = STAGE ? scr + X::T::template scratch<HALF>() : nullptr;
-  for (int base = 0; base < N; base += NTEAM) {
-    const int kx = base + team;
-    const bool act = kx < N;
-    if (!__any_sync(0xffffffffu, act)) continue;
-    if constexpr (STAGE) {
-      if (act && a.fold) {
-        constexpr int E = 16 / sizeof(C);   // elements per 16-byte chunk
-        const C* row = Q + (size_t)(kx < N / 2 ? kx : N - 1 - kx) * QW;
-        for (int c = g; c < (N / 2) / E; c += G) cp_async16(qb + c * E, row + c * E);
-      }
-      cp_async_commit();
-    }
-    C v[RR];
-#pragma unroll
-    for (int r = 0; r < RR; ++r) {
-      v[r] = czero<C>();
-      if (r < NZ && r < rv) {
-        const int y = g + G * r;
-        if (act && y < nby) v[r] = M[y * P + kx];
-      }
-    }
-    X::T::template forward<NZ, HALF>(v, tw, scr, g);
-    if constexpr (STAGE) {
-      cp_async_wait_all();
-      __syncwarp();
-    }
-    if (act) {
-      if (a.fold) {
-        // bins k and N-1-k share a phasor; ky = g*CC + j + RR*q < N/2 exactly when q < G/2
-        const C* Qrow = STAGE ? qb : Q + (size_t)(kx < N / 2 ? kx : N - 1 - kx) * QW;
-#pragma unroll
-        for (int j = 0; j < CC; ++j)
-#pragma unroll
-          for (int q = 0; q < G; ++q) {
-            const int ky = g * CC + j + RR * q;
-            v[j * G + q] = cmul(v[j * G + q], Qrow[q < G / 2 ? ky : N - 1 - ky]);
-          }
-      } else {
-        const C* Qrow = Q + (size_t)kx * QW;
-#pragma unroll
-        for (int j = 0; j < CC; ++j)
-#pragma unroll
-          for (int q = 0; q < G; ++q) v[j * G + q] = cmul(v[j * G + q], Qrow[g * CC + j + RR * q]);
-      }
-    }
-    // (the inverse's exchange syncs the warp: every lane has read the buffer
-    // before the next task's copies overwrite it)
-    X::T::template inverse<HALF>(v, tw, scr, g);
-    if (act) {
-#pragma unroll
-      for (int r = 0; r < RR; ++r) {
-        if (r < NZ && r < rv) {
-          const int y = g + G * r;
-          if (y < nby) M[y * P + kx] = v[r];
-        }
-      }
-    }
-  }
-  __syncthreads();
-}
-
-// Phase 3: inverse FFT along x of every box row, tilt/surface map, then the
-// epilogue: store the propagated field into obuf (first of two propagations)
-// or apply the boundary mix and write the new (masked) fields.
-template <typename C, int N, bool MIX, int NZ, int NT, bool HALF = false>
-__device__ __forceinline__ void fused_phase3(const FusedArgs<C>& a, const StepDesc& sd, int f, int region,
-                                             bool prop_is_b, C* M, C* scr, C* obuf,
-                                             const C* tw, int team, int g) {
-  using X = FusedCtx<C, N>;
-  constexpr int G = X::G, RR = X::RR, CC = X::CC, P = X::P;
-  constexpr int NTEAM = NT;
-  const int nbx = a.nbx, nby = a.nby;
-  const size_t plane = (size_t)nby * nbx;
-  const int ti = a.tilt_idx[region];
-  const C* tmap = ti >= 0 ? a.tilt + ((size_t)f * a.ntilt + ti) * plane : nullptr;
-  C* stA = sd.sa >= 0 ? a.state + ((size_t)f * a.nslots + sd.sa) * plane : nullptr;
-  C* stB = sd.sb >= 0 ? a.state + ((size_t)f * a.nslots + sd.sb) * plane : nullptr;
-  const C* add = (MIX && sd.addA >= 0) ? a.addbuf + (size_t)sd.addA * plane : nullptr;
-  const int rv = (nbx + G - 1) / G;
-  C cAA, cAB, cBA, cBB;
-  if (MIX) {
-    const double2* cf = a.coefs + 4 * sd.coef;
-    cAA = from_d<C>(cf[0]); cAB = from_d<C>(cf[1]); cBA = from_d<C>(cf[2]); cBB = from_d<C>(cf[3]);
-  }
-  for (int base = 0; base < nby; base += NTEAM) {
-    const int y = base + team;
-    const bool act = y < nby;
-    if (!__any_sync(0xffffffffu, act)) continue;
-    C v[RR];
-#pragma unroll
-    for (int j = 0; j < CC; ++j)
-#pragma unroll
-      for (int q = 0; q < G; ++q) v[j * G + q] = act ? M[y * P + g * CC + j + RR * q] : czero<C>();
-    X::T::template inverse<HALF>(v, tw, scr, g);
-    if (!act) continue;
-#pragma unroll
-    for (int r = 0; r < RR; ++r) {
-      if (r >= NZ || r >= rv) continue;
-      const int x = g + G * r;
-      if (x >= nbx) continue;
-      const int i = y * nbx + x;
-      C p = v[r];
-      if (tmap) p = cmul(p, tmap[i]);
-      if (!MIX) {
-        obuf[i] = p;
-      } else {
-        // new fields are stored masked (their next propagation masks them anyway)
-        const bool in = a.mask[i] != 0;
-        C tA, tB;
-        if (prop_is_b) {
-          tB = p;
-          if (sd.ra >= 0) tA = obuf[i];
-          else tA = stA ? stA[i] : czero<C>();
-        } else {
-          tA = p;
-          tB = stB ? stB[i] : czero<C>();
-        }
-        if (stA) {
-          C o = cadd(cmul(cAA, tA), cmul(cAB, tB));
-          if (add) o = cadd(o, add[i]);
-          stA[i] = in ? o : czero<C>();
-        }
-        if (stB) stB[i] = in ? cadd(cmul(cBA, tA), cmul(cBB, tB)) : czero<C>();
-      }
-    }
-  }
-}
-
-// ---- joint step: both slots processed together ------------------------------
-// The rows of A and of B form one task list (2 nby rows), and so do their
-// columns (2 N), so the teams stay busy where a single field's nby rows leave
-// most of them idle in the last round; the propagated fields stay in the row
-// tiles MA, MB and the boundary mix runs as one pass over the box.  A team
-// takes the tasks t0 + team, t0 + team + ts, ... (the fused kernel: t0 = 0,
-// ts = its teams; the split-phase kernels spread the tasks over CTAs); the
-// tasks of a slot that is not propagated (pa / pb false) are skipped.
-
-// Phase 1, joint: forward FFT along x of the box rows of A (tasks < nby) and B.
-template <typename C, int N, int NZ, int NT, bool SPLIT, bool HALF = false>
-__device__ __forceinline__ void joint_phase1(const FusedArgs<C>& a, const StepDesc& sd, int f, C* MA, C* MB,
-                                             C* scr, const C* tw, int team, int g, int t0, int ts,
-                                             bool pa, bool pb) {
-  using X = FusedCtx<C, N>;
-  constexpr int G = X::G, RR = X::RR, CC = X::CC, P = X::P;
-  const int nbx = a.nbx, nby = a.nby, ntask = 2 * nby;
-  const int rv = (nbx + G - 1) / G;
-  // the fused kernel's joint steps: all tasks of the CTA, both slots propagated
-  const int T0 = SPLIT ? t0 : 0, TS = SPLIT ? ts : NT;
-  for (int base = T0; base < ntask; base += TS) {
-    const int t = base + team;
-    const bool act = t < ntask && (!SPLIT || (t >= nby ? pb : pa));
-    if (!__any_sync(0xffffffffu, act)) continue;
-    const bool isb = act && t >= nby;
-    const int y = act ? (isb ? t - nby : t) : 0;
-    const int slot = isb ? sd.sb : sd.sa, exitk = isb ? sd.exitB : sd.exitA;
-    const C* row = a.state + (((size_t)f * a.nslots + slot) * nby + y) * (size_t)nbx;
-    double2* arow = exitk >= 0 ? a.exitacc + (((size_t)exitk * a.nfreq + f) * nby + y) * (size_t)nbx : nullptr;
-    C v[RR];
-#pragma unroll
-    for (int r = 0; r < RR; ++r) {
-      v[r] = czero<C>();
-      if (r < NZ && r < rv) {
-        const int x = g + G * r;
-        if (act && x < nbx) {
-          const C val = row[x];
-          v[r] = val;
-          if (arow) {
-            double2 o = arow[x];
-            double2 d = to_d(val);
-            arow[x] = make_double2(o.x + d.x, o.y + d.y);
-          }
-        }
-      }
-    }
-    X::T::template forward<NZ, HALF>(v, tw, scr, g);
-    if (act) {
-      C* M = isb ? MB : MA;
-#pragma unroll
-      for (int j = 0; j < CC; ++j)
-#pragma unroll
-        for (int q = 0; q < G; ++q) M[y * P + g * CC + j + RR * q] = v[j * G + q];
-    }
-  }
-  __syncthreads();
-}
-
-// Ask L2 for the phasor row of column task t (rows of 128-byte lines, one per
-// thread g of the team), so that it is there when the team reaches that task.
-// QA / QB are null for a slot that is not propagated.
-template <typename C, int N, bool MAYBE_NULL>
-__device__ __forceinline__ void prefetch_qrow(const FusedArgs<C>& a, const C* QA, const C* QB, int t, int g) {
-  if (t >= 2 * N) return;
-  const int QW = a.fold ? N / 2 : N;
-  const int kx = t < N ? t : t - N;
-  const C* Q = t < N ? QA : QB;
-  if (MAYBE_NULL && !Q) return;
-  const C* row = Q + (size_t)(a.fold ? (kx < N / 2 ? kx : N - 1 - kx) : kx) * QW;
-  const int lines = (int)((sizeof(C) * QW + 127) / 128);
-  if (g < lines) asm volatile("prefetch.global.L2 [%0];" ::"l"(reinterpret_cast<const char*>(row) + 128 * g));
-}
-
-// Phase 2, joint: columns of A (tasks < N) and of B, each with its region's phasor.
-// STAGE as fused_phase2 (the fused kernel only).
-template <typename C, int N, int NZ, int NT, bool SPLIT, bool HALF = false, bool STAGE = false>
-__device__ __forceinline__ void joint_phase2(const FusedArgs<C>& a, const C* QA, const C* QB, C* MA, C* MB, C* scr,
-                                             const C* tw, int team, int g, int t0, int ts) {
-  using X = FusedCtx<C, N>;
-  constexpr int G = X::G, RR = X::RR, CC = X::CC, P = X::P;
-  static_assert(!(SPLIT && STAGE), "staged phasor rows: fused kernel only");
-  const int nby = a.nby;
-  const int QW = a.fold ? N / 2 : N;
-  const int rv = (nby + G - 1) / G;
-  const int T0 = SPLIT ? t0 : 0, TS = SPLIT ? ts : NT;
-  C* qb = STAGE ? scr + X::T::template scratch<HALF>() : nullptr;
-  for (int base = T0; base < 2 * N; base += TS) {
-    const int t = base + team;
-    const bool act = t < 2 * N && (!SPLIT || (t >= N ? QB : QA) != nullptr);
-    if (!__any_sync(0xffffffffu, act)) continue;
-    const bool isb = act && t >= N;
-    const int kx = act ? (isb ? t - N : t) : 0;
-    C* M = isb ? MB : MA;
-    const C* Q = isb ? QB : QA;
-    if constexpr (STAGE) {
-      if (act && a.fold) {
-        constexpr int E = 16 / sizeof(C);   // elements per 16-byte chunk
-        const C* row = Q + (size_t)(kx < N / 2 ? kx : N - 1 - kx) * QW;
-        for (int c = g; c < (N / 2) / E; c += G) cp_async16(qb + c * E, row + c * E);
-      }
-      cp_async_commit();
-      if (!a.fold) prefetch_qrow<C, N, SPLIT>(a, QA, QB, t + TS, g);
-    } else {
-      prefetch_qrow<C, N, SPLIT>(a, QA, QB, t + TS, g);
-    }
-    C v[RR];
-#pragma unroll
-    for (int r = 0; r < RR; ++r) {
-      v[r] = czero<C>();
-      if (r < NZ && r < rv) {
-        const int y = g + G * r;
-        if (act && y < nby) v[r] = M[y * P + kx];
-      }
-    }
-    X::T::template forward<NZ, HALF>(v, tw, scr, g);
-    if constexpr (STAGE) {
-      cp_async_wait_all();
-      __syncwarp();
-    }
-    if (act) {
-      if (a.fold) {
-        const C* Qrow = STAGE ? qb : Q + (size_t)(kx < N / 2 ? kx : N - 1 - kx) * QW;
-#pragma unroll
-        for (int j = 0; j < CC; ++j)
-#pragma unroll
-          for (int q = 0; q < G; ++q) {
-            const int ky = g * CC + j + RR * q;
-            v[j * G + q] = cmul(v[j * G + q], Qrow[q < G / 2 ? ky : N - 1 - ky]);
-          }
-      } else {
-        const C* Qrow = Q + (size_t)kx * QW;
-#pragma unroll
-        for (int j = 0; j < CC; ++j)
-#pragma unroll
-          for (int q = 0; q < G; ++q) v[j * G + q] = cmul(v[j * G + q], Qrow[g * CC + j + RR * q]);
-      }
-    }
-    // (the inverse's exchange syncs the warp before the buffer is refilled)
-    X::T::template inverse<HALF>(v, tw, scr, g);
-    if (act) {
-#pragma unroll
-      for (int r = 0; r < RR; ++r) {
-        if (r < NZ && r < rv) {
-          const int y = g + G * r;
-          if (y < nby) M[y * P + kx] = v[r];
-        }
-      }
-    }
-  }
-  __syncthreads();
-}
-
-// Phase 3, joint: inverse FFT along x of the box rows of A and B, times the
-// region's tilt/surface map, written back in place into the row's first nbx
-// entries (the team's exchange has already consumed the row).
-template <typename C, int N, int NZ, int NT, bool SPLIT, bool HALF = false>
-__device__ __forceinline__ void joint_phase3(const FusedArgs<C>& a, const StepDesc& sd, int f, C* MA, C* MB,
-                                             C* scr, const C* tw, int team, int g, int t0, int ts,
-                                             bool pa, bool pb) {
-  using X = FusedCtx<C, N>;
-  constexpr int G = X::G, RR = X::RR, CC = X::CC, P = X::P;
-  const int nbx = a.nbx, nby = a.nby, ntask = 2 * nby;
-  const size_t plane = (size_t)nby * nbx;
-  const int tiA = (!SPLIT || pa) ? a.tilt_idx[sd.ra] : -1, tiB = (!SPLIT || pb) ? a.tilt_idx[sd.rb] : -1;
-  const C* tA = tiA >= 0 ? a.tilt + ((size_t)f * a.ntilt + tiA) * plane : nullptr;
-  const C* tB = tiB >= 0 ? a.tilt + ((size_t)f * a.ntilt + tiB) * plane : nullptr;
-  const int rv = (nbx + G - 1) / G;
-  const int T0 = SPLIT ? t0 : 0, TS = SPLIT ? ts : NT;
-  for (int base = T0; base < ntask; base += TS) {
-    const int t = base + team;
-    const bool act = t < ntask && (!SPLIT || (t >= nby ? pb : pa));
-    if (!__any_sync(0xffffffffu, act)) continue;
-    const bool isb = act && t >= nby;
-    const int y = act ? (isb ? t - nby : t) : 0;
-    C* M = isb ? MB : MA;
-    const C* tmap = isb ? tB : tA;
-    C v[RR];
-#pragma unroll
-    for (int j = 0; j < CC; ++j)
-#pragma unroll
-      for (int q = 0; q < G; ++q) v[j * G + q] = act ? M[y * P + g * CC + j + RR * q] : czero<C>();
-    X::T::template inverse<HALF>(v, tw, scr, g);
-    if (!act) continue;
-#pragma unroll
-    for (int r = 0; r < RR; ++r) {
-      if (r >= NZ || r >= rv) continue;
-      const int x = g + G * r;
-      if (x >= nbx) continue;
-      C p = v[r];
-      if (tmap) p = cmul(p, tmap[y * nbx + x]);
-      M[y * P + x] = p;
-    }
-  }
-  __syncthreads();
-}
-
-// Boundary mix of a step over the box: A' = cAA A~ + cAB B~ (+ add),
-// B' = cBA A~ + cBB B~, stored masked; X~ is the propagated field (row tile)
-// of a propagated slot, else the slot's stored field.  Pixels i0, i0 + is, ...
-template <typename C, int N>
-__device__ __forceinline__ void joint_mix(const FusedArgs<C>& a, const StepDesc& sd, int f, const C* MA,
-                                          const C* MB, bool pa, bool pb, int i0, int is) {
-  constexpr int P = FusedCtx<C, N>::P;
-  const int nbx = a.nbx, nby = a.nby;
-  const size_t plane = (size_t)nby * nbx;
-  C* stA = sd.sa >= 0 ? a.state + ((size_t)f * a.nslots + sd.sa) * plane : nullptr;
-  C* stB = sd.sb >= 0 ? a.state + ((size_t)f * a.nslots + sd.sb) * plane : nullptr;
-  const C* add = sd.addA >= 0 ? a.addbuf + (size_t)sd.addA * plane : nullptr;
-  const double2* cf = a.coefs + 4 * sd.coef;
-  const C cAA = from_d<C>(cf[0]), cAB = from_d<C>(cf[1]), cBA = from_d<C>(cf[2]), cBB = from_d<C>(cf[3]);
-  for (int i = i0; i < (int)plane; i += is) {
-    const int y = i / nbx, x = i - y * nbx;
-    const C A = pa ? MA[y * P + x] : (stA ? stA[i] : czero<C>());
-    const C B = pb ? MB[y * P + x] : (stB ? stB[i] : czero<C>());
-    const bool in = a.mask[i] != 0;
-    if (stA) {
-      C o = cadd(cmul(cAA, A), cmul(cAB, B));
-      if (add) o = cadd(o, add[i]);
-      stA[i] = in ? o : czero<C>();
-    }
-    if (stB) stB[i] = in ? cadd(cmul(cBA, A), cmul(cBB, B)) : czero<C>();
-  }
-}
-
-// One bounce stage: grid = (steps of the stage, frequencies).  JOINT: steps
-// with both slots propagated take the joint path (twice the row tile in
-// shared memory).  NZ: box lines occupy at most NZ of a thread's RR register
-// slots (x = g + G r < nbx, y = g + G r < nby only for r < NZ), so the first
-// forward pass is pruned and the inverse stores only NZ slots.  MINB: CTAs
-// per SM the registers are sized for.  MODE: kModeTwShared | kModeHalf |
-// kModeStage (fewer registers or less shared memory per warp, so more warps
-// per SM, and phasor rows staged ahead); the arithmetic, and so every result,
-// is the same.
-template <typename R, int N, bool JOINT, int NZ, int THREADS, int MINB, int MODE>
-__global__ void __launch_bounds__(THREADS, MINB) k_fused_stage(FusedArgs<cplx_t<R>> a) {
-  using C = cplx_t<R>;
-  using X = FusedCtx<C, N>;
-  constexpr int G = X::G, RR = X::RR, P = X::P;
-  constexpr int NTEAM = THREADS / G;
-  extern __shared__ __align__(128) unsigned char smem_raw[];
-  const int nby = a.nby;
-  C* M = reinterpret_cast<C*>(smem_raw + kSmemHeader);
-  C* scr_all = M + (JOINT ? 2 : 1) * nby * P;
-  const int tid = threadIdx.x, team = tid / G, g = tid % G;
-  constexpr bool HALF = (MODE & kModeHalf) != 0, STAGE = (MODE & kModeStage) != 0;
-  C* scr = scr_all + team * team_region<N, MODE>();
-  const StepDesc sd = a.steps[blockIdx.x];
-  const int f = blockIdx.y;
-  C twr[RR];
-  const C* tw = twr;
-  if constexpr ((MODE & kModeTwShared) != 0) {
-    // tw[g][s] = W_N^(g s) behind the teams' regions, rows RR + 1 apart so
-    // that the G threads of a team reading their s-th twiddle hit distinct banks
-    C* tws = scr_all + NTEAM * team_region<N, MODE>();
-    for (int i = tid; i < G * RR; i += THREADS)
-      tws[(i / RR) * (RR + 1) + i % RR] = root1024<C>((i / RR) * (i % RR) * (1024 / N));
-    __syncthreads();
-    tw = tws + g * (RR + 1);
-  } else {
-    team_twiddles<N>(twr, g);
-  }
-  const int QW = a.fold ? N / 2 : N;
-  auto qptr = [&](int region) -> const C* {
-    return a.phasor + ((size_t)f * a.ntab + region) * (size_t)(QW * QW);
-  };
-  const bool pa = sd.ra >= 0, pb = sd.rb >= 0;
-  if (JOINT && pa && pb) {
-    C* MB = M + nby * P;
-    prefetch_qrow<C, N, false>(a, qptr(sd.ra), qptr(sd.rb), team, g);
-    joint_phase1<C, N, NZ, NTEAM, false, HALF>(a, sd, f, M, MB, scr, tw, team, g, 0, NTEAM, true, true);
-    joint_phase2<C, N, NZ, NTEAM, false, HALF, STAGE>(a, qptr(sd.ra), qptr(sd.rb), M, MB, scr, tw, team, g, 0,
-                                                      NTEAM);
-    joint_phase3<C, N, NZ, NTEAM, false, HALF>(a, sd, f, M, MB, scr, tw, team, g, 0, NTEAM, true, true);
-    joint_mix<C, N>(a, sd, f, M, MB, true, true, threadIdx.x, blockDim.x);
-  } else if (pa && pb) {
-    // A~ is parked in the A slot itself until the boundary mix
-    C* obuf = a.state + ((size_t)f * a.nslots + sd.sa) * (size_t)(nby * a.nbx);
-    fused_phase1<C, N, NZ, NTEAM, HALF>(a, f, sd.sa, sd.exitA, M, scr, tw, team, g);
-    fused_phase2<C, N, NZ, NTEAM, HALF, STAGE>(a, qptr(sd.ra), M, scr, tw, team, g);
-    fused_phase3<C, N, false, NZ, NTEAM, HALF>(a, sd, f, sd.ra, false, M, scr, obuf, tw, team, g);
-    // no barrier: B's forward row pass writes row y of M through the same
-    // team (y mod NTEAM) and the same per-thread elements that A's inverse row
-    // pass just read from it, and A~ goes to global memory, read back in B's
-    // mix by the same thread; program order already orders every access
-    fused_phase1<C, N, NZ, NTEAM, HALF>(a, f, sd.sb, sd.exitB, M, scr, tw, team, g);
-    fused_phase2<C, N, NZ, NTEAM, HALF, STAGE>(a, qptr(sd.rb), M, scr, tw, team, g);
-    fused_phase3<C, N, true, NZ, NTEAM, HALF>(a, sd, f, sd.rb, true, M, scr, obuf, tw, team, g);
-  } else if (pa) {
-    fused_phase1<C, N, NZ, NTEAM, HALF>(a, f, sd.sa, sd.exitA, M, scr, tw, team, g);
-    fused_phase2<C, N, NZ, NTEAM, HALF, STAGE>(a, qptr(sd.ra), M, scr, tw, team, g);
-    fused_phase3<C, N, true, NZ, NTEAM, HALF>(a, sd, f, sd.ra, false, M, scr, nullptr, tw, team, g);
-  } else if (pb) {
-    fused_phase1<C, N, NZ, NTEAM, HALF>(a, f, sd.sb, sd.exitB, M, scr, tw, team, g);
-    fused_phase2<C, N, NZ, NTEAM, HALF, STAGE>(a, qptr(sd.rb), M, scr, tw, team, g);
-    fused_phase3<C, N, true, NZ, NTEAM, HALF>(a, sd, f, sd.rb, true, M, scr, nullptr, tw, team, g);
-  }
-}
-
-// ---- split-phase stage: for stages with fewer steps x frequencies than SMs --
-// The four phases of a step (forward rows, columns, inverse rows, boundary
-// mix) run as four launches whose tasks are spread over blockIdx.z, so a
-// stage with a handful of steps (one frequency, a short stack) still spreads
-// its FFT work over many SMs.  The row tiles of step s, frequency f live in
-// global memory at a.mg + (s nfreq + f) 2 nby P (A, then B) and stay in L2.
-constexpr int kSplitThreads = 64;
-
-template <typename R, int N, int NZ>
-__global__ void __launch_bounds__(kSplitThreads) k_split_phase(FusedArgs<cplx_t<R>> a, int phase) {
-  using C = cplx_t<R>;
-  using X = FusedCtx<C, N>;
-  constexpr int G = X::G, RR = X::RR, P = X::P;
-  extern __shared__ __align__(128) unsigned char smem_raw[];
-  const int tid = threadIdx.x, team = tid / G, g = tid % G, nteam = blockDim.x / G;
-  // programmatic dependent launch: let the next phase launch now, and wait for
-  // the previous phase (its writes visible) before reading anything it wrote
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-  C tw[RR];
-  team_twiddles<N>(tw, g);
-  asm volatile("griddepcontrol.wait;" ::: "memory");
-  const StepDesc sd = a.steps[blockIdx.x];
-  const int f = blockIdx.y;
-  C* MA = a.mg + ((size_t)blockIdx.x * a.nfreq + f) * 2 * (size_t)a.nby * P;
-  C* MB = MA + (size_t)a.nby * P;
-  const bool pa = sd.ra >= 0, pb = sd.rb >= 0;
-  if (phase == 3) {
-    joint_mix<C, N>(a, sd, f, MA, MB, pa, pb, blockIdx.z * blockDim.x + tid, gridDim.z * blockDim.x);
-    return;
-  }
-  C* scr = reinterpret_cast<C*>(smem_raw) + team * X::T::SCR;
-  const int t0 = blockIdx.z * nteam, ts = gridDim.z * nteam;
-  if (phase == 0) {
-    joint_phase1<C, N, NZ, kSplitThreads / G, true>(a, sd, f, MA, MB, scr, tw, team, g, t0, ts, pa, pb);
-  } else if (phase == 1) {
-    const int QW = a.fold ? N / 2 : N;
-    const C* QA = pa ? a.phasor + ((size_t)f * a.ntab + sd.ra) * (size_t)(QW * QW) : nullptr;
-    const C* QB = pb ? a.phasor + ((size_t)f * a.ntab + sd.rb) * (size_t)(QW * QW) : nullptr;
-    joint_phase2<C, N, NZ, kSplitThreads / G, true>(a, QA, QB, MA, MB, scr, tw, team, g, t0, ts);
-  } else {
-    joint_phase3<C, N, NZ, kSplitThreads / G, true>(a, sd, f, MA, MB, scr, tw, team, g, t0, ts, pa, pb);
-  }
-}
 
 static int sm_count() {
   static int n = 0;
@@ -734,54 +129,25 @@ static int sm_count() {
   return n;
 }
 
-template <typename R, int N, int NZ>
-static int launch_split(const FusedArgs<cplx_t<R>>& a, int nsteps, cudaStream_t st) {
-  using T = Team<N>;
-  const int nteam = kSplitThreads / T::G;
-  const size_t smem = sizeof(cplx_t<R>) * nteam * T::SCR;
-  const int zr = (2 * a.nby + nteam - 1) / nteam, zc = (2 * N + nteam - 1) / nteam;
-  const int zm = (a.nbx * a.nby + kSplitThreads - 1) / kSplitThreads;
-  const int z[4] = {zr, zc, zr, zm};
-  // each phase may launch while the previous one drains (programmatic
-  // dependent launch); the kernel waits for it before touching its data
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  for (int ph = 0; ph < 4; ++ph) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(nsteps, a.nfreq, z[ph]);
-    cfg.blockDim = dim3(kSplitThreads);
-    cfg.dynamicSmemBytes = ph == 3 ? 0 : smem;
-    cfg.stream = st;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    COUNT_LAUNCH();
-    const cudaError_t e = cudaLaunchKernelEx(&cfg, k_split_phase<R, N, NZ>, a, ph);
-    if (e != cudaSuccess) return (int)e;
-  }
-  return 0;
-}
+// Whether stages of this transform length may take the split-phase path.
+bool split_length(int N) { return N >= 40; }
 
 // Bytes of the split-phase row tiles for a stage of `nsteps` steps.
 size_t split_tile_bytes(int N, int nby, int nfreq, int nsteps, bool fp64) {
-  return (size_t)nsteps * nfreq * 2 * nby * (N + 2) * (fp64 ? 16 : 8);
+  return (size_t)nsteps * nfreq * 2 * nby * pitch_of(N) * (fp64 ? 16 : 8);
 }
 
 // Whether a stage of `nsteps` steps x `nfreq` frequencies takes the split path.
 bool split_stage(int nsteps, int nfreq) { return (long long)nsteps * nfreq < sm_count(); }
-
-template <int N, int MODE = 0>
-static size_t fused_smem_for(int nby, size_t csz, int tiles = 1, int threads = kFusedThreads) {
-  const size_t nteam = threads / Team<N>::G;
-  const size_t twt = (MODE & kModeTwShared) ? (size_t)Team<N>::G * (Team<N>::RR + 1) : 0;   // twiddle table
-  return kSmemHeader + csz * ((size_t)tiles * nby * fused_pitch<N>() + nteam * team_region<N, MODE>() + twt);
-}
 
 static size_t smem_for(int N, int nby, size_t csz) {
   switch (N) {
     case 8: return fused_smem_for<8>(nby, csz);
     case 16: return fused_smem_for<16>(nby, csz);
     case 32: return fused_smem_for<32>(nby, csz);
+    case 40: return fused_smem_for<40>(nby, csz, 1, 96);
+    case 80: return fused_smem_for<80, kModeTwShared>(nby, csz, 1, 160);
+    case 160: return fused_smem_for<160, kModeTwShared>(nby, csz, 1, 320);
     case 64: return fused_smem_for<64>(nby, csz);
     case 128: return fused_smem_for<128>(nby, csz);
     case 256: return fused_smem_for<256>(nby, csz);
@@ -789,46 +155,28 @@ static size_t smem_for(int N, int nby, size_t csz) {
   }
 }
 
-static const size_t kMaxSmem = 227 * 1024;
-
 size_t fused_smem_bytes(int N, int nbx, int nby, bool fp64) {
   (void)nbx;
   return smem_for(N, nby, fp64 ? 16 : 8);
 }
 
 bool fused_split_only(int N, int nbx, int nby, bool fp64) {
-  return N >= 64 && fused_smem_bytes(N, nbx, nby, fp64) > kMaxSmem;
+  return split_length(N) && fused_smem_bytes(N, nbx, nby, fp64) > kMaxSmem;
 }
 
 bool fused_supported(int N, int nbx, int nby, bool fp64) {
-  if (N < 8 || N > 256 || (N & (N - 1))) return false;
+  const bool five = N == 80 || (!fp64 && (N == 40 || N == 160));
+  if (N < 8 || N > 256 || ((N & (N - 1)) && !five)) return false;
   if (nbx < 1 || nby < 1 || nbx > N || nby > N) return false;
   // row tiles too large for shared memory (complex128 at 256^2): every stage
   // takes the split-phase path, whose tiles live in global memory
   return fused_smem_bytes(N, nbx, nby, fp64) <= kMaxSmem || fused_split_only(N, nbx, nby, fp64);
 }
 
-// Shared memory of one SM (bytes) and what the driver reserves per CTA.
-static const size_t kSmemPerSM = 228 * 1024, kSmemReservedPerCta = 1024;
-
-// The dynamic shared-memory limit of a kernel is raised to the per-block
-// maximum, the same value for every launch: launches of one kernel with
-// different sizes from several host threads (the serving engine's workers)
-// must not lower it under one another.
-template <typename R, int N, bool JOINT, int NZ, int THREADS = kFusedThreads,
-          int MINB = (sizeof(R) == 4 && N <= 128) ? 2 : 1, int MODE = 0>
-static int launch_fused_v(const FusedArgs<cplx_t<R>>& a, dim3 grid, size_t smem, cudaStream_t st) {
-  cudaError_t e = cudaFuncSetAttribute(k_fused_stage<R, N, JOINT, NZ, THREADS, MINB, MODE>,
-                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxSmem);
-  if (e != cudaSuccess) return (int)e;
-  k_fused_stage<R, N, JOINT, NZ, THREADS, MINB, MODE><<<grid, THREADS, smem, st>>>(a);
-  return (int)cudaGetLastError();
-}
-
 // Register slots a box line may occupy in the pruned variants (complex64 for
-// N >= 64, complex128 for N = 64, 128): 5 of 16 (3 of 8) covers boxes up to
-// 5/16 of the grid, the disk of radius 0.15 m in the reference's 1 m window.
-template <int N> constexpr int pruned_slots() { return (5 * Team<N>::RR + 15) / 16; }
+// N >= 64, complex128 for N = 64, 128): half of them, since a transform of the
+// truncated kernel (compact_length) is at least twice as long as the box.
+template <int N> constexpr int pruned_slots() { return Team<N>::RR / 2; }
 
 // Shape of one fused-stage launch: shared memory of the single and doubled
 // (joint) row tiles and whether the rule takes the joint path.
@@ -896,6 +244,9 @@ std::vector<int> fused_variants(int N, int nbx, int nby, bool fp64) {
     case 8: return fused_variants_t<8>(nbx, nby, fp64);
     case 16: return fused_variants_t<16>(nbx, nby, fp64);
     case 32: return fused_variants_t<32>(nbx, nby, fp64);
+    case 40:
+    case 80:
+    case 160: return fp64 ? five_variants_d(N, nby) : five_variants_f(N, nby);
     case 64: return fused_variants_t<64>(nbx, nby, fp64);
     case 128: return fused_variants_t<128>(nbx, nby, fp64);
     case 256: return fused_variants_t<256>(nbx, nby, fp64);
@@ -969,6 +320,11 @@ static int launch_fused_dispatch(int N, const FusedArgs<cplx_t<R>>& a, int nstep
     case 8: return launch_fused_t<R, 8>(a, nsteps, st);
     case 16: return launch_fused_t<R, 16>(a, nsteps, st);
     case 32: return launch_fused_t<R, 32>(a, nsteps, st);
+    case 40:
+    case 80:
+    case 160:
+      if constexpr (sizeof(R) == 4) return launch_five_f(N, a, nsteps, st);
+      else return launch_five_d(N, a, nsteps, st);
     case 64: return launch_fused_t<R, 64>(a, nsteps, st);
     case 128: return launch_fused_t<R, 128>(a, nsteps, st);
     case 256: return launch_fused_t<R, 256>(a, nsteps, st);
@@ -987,7 +343,7 @@ int launch_fused_stage_d(int N, const FusedArgs<double2>& a, int nsteps, cudaStr
 // Phasor and tilt tables
 // ---------------------------------------------------------------------------
 template <typename C>
-__global__ void k_phasor_table(C* out, int nfreq, const double* freqs, int ntab, const int* regions,
+__global__ void k_phasor_table(C* out, const double* freqs, int stride, const int* regions,
                                const RegionGeo* geo, int N, const double* kX, const double* kY,
                                int fold) {
   const int W = fold ? N / 2 : N;
@@ -1002,18 +358,155 @@ __global__ void k_phasor_table(C* out, int nfreq, const double* freqs, int ntab,
   const double2 k0 = k0_of(lambda, gg.eps_re, gg.eps_im);
   double2 v = phasor_value(k0, kX[sx], kY[sy], gg.dz);
   const double sc = 1.0 / ((double)N * (double)N);   // a power of two: exact
-  out[((size_t)f * ntab + t) * per + idx] = from_d_phase<C>(make_double2(v.x * sc, v.y * sc));
+  out[((size_t)f * stride + t) * per + idx] = from_d_phase<C>(make_double2(v.x * sc, v.y * sc));
 }
 
-int launch_phasor_table(bool fp64, void* out, int nfreq, const double* d_freqs, int ntab,
+int launch_phasor_table(bool fp64, void* out, int nfreq, const double* d_freqs, int ntab, int stride,
                         const int* d_regions, const RegionGeo* d_geo, int N, const double* d_kX,
                         const double* d_kY, int fold, cudaStream_t st) {
   if (ntab <= 0 || nfreq <= 0) return 0;
   const int W = fold ? N / 2 : N;
   dim3 grid((W * W + 255) / 256, ntab, nfreq);
-  if (fp64) { COUNT_LAUNCH(); k_phasor_table<double2><<<grid, 256, 0, st>>>((double2*)out, nfreq, d_freqs, ntab, d_regions, d_geo, N, d_kX, d_kY, fold); }
-  else { COUNT_LAUNCH(); k_phasor_table<float2><<<grid, 256, 0, st>>>((float2*)out, nfreq, d_freqs, ntab, d_regions, d_geo, N, d_kX, d_kY, fold); }
+  if (fp64) { COUNT_LAUNCH(); k_phasor_table<double2><<<grid, 256, 0, st>>>((double2*)out, d_freqs, stride, d_regions, d_geo, N, d_kX, d_kY, fold); }
+  else { COUNT_LAUNCH(); k_phasor_table<float2><<<grid, 256, 0, st>>>((float2*)out, d_freqs, stride, d_regions, d_geo, N, d_kX, d_kY, fold); }
   return (int)cudaGetLastError();
+}
+
+// Spectrum of the truncated kernel (see compact_length) of one (frequency,
+// region) per CTA: S = Ax^T D Ay over one quadrant, D the N x N grid's phasors
+// at the non-negative wavenumbers and A the real matrix of compact_matrix
+// (weights, both cosine sums and all scales included).  blockIdx.z takes a
+// slice of BS columns of S.  Rows of D are evaluated kChunk at a time, reduced
+// to BS columns, and added to the CTA's S in registers (E per thread).
+// Bound by the FP64 pipe (2 FMA per clock and SM): for N = 128 to length 80 a
+// table takes 4096 phasors and 532k real FMAs, about equal shares; operands
+// come from L1 and shared memory far faster than that.
+constexpr int kChunk = 16;
+template <typename C, int E>
+__global__ void __launch_bounds__(256) k_compact_table(C* out, const double* freqs, int stride, const int* regions,
+                                                       const RegionGeo* geo, int Q, int first, const double* kX,
+                                                       const double* kY, const double* A, int H, int BS) {
+  extern __shared__ __align__(16) unsigned char sm[];
+  double2* D = reinterpret_cast<double2*>(sm);   // [kChunk][Q]
+  double2* T = D + kChunk * Q;                   // [kChunk][BS]
+  const int tid = threadIdx.x, b0 = blockIdx.z * BS;
+  const RegionGeo gg = geo[regions[blockIdx.x]];
+  const double2 k0 = k0_of(SPEED_OF_LIGHT / freqs[blockIdx.y], gg.eps_re, gg.eps_im);
+  double2 s[E];
+#pragma unroll
+  for (int i = 0; i < E; ++i) s[i] = make_double2(0.0, 0.0);
+  for (int x0 = 0; x0 < Q; x0 += kChunk) {
+    const int nx = min(kChunk, Q - x0);
+    for (int i = tid; i < nx * Q; i += 256)
+      D[i] = phasor_value(k0, kX[first + x0 + i / Q], kY[first + i % Q], gg.dz);
+    __syncthreads();
+    for (int i = tid; i < nx * BS; i += 256) {
+      const int r = i / BS, b = i % BS;
+      double2 t = make_double2(0.0, 0.0);
+      for (int q = 0; q < Q; ++q) {
+        const double w = A[q * H + b0 + b];
+        const double2 d = D[r * Q + q];
+        t.x = fma(d.x, w, t.x);
+        t.y = fma(d.y, w, t.y);
+      }
+      T[i] = t;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < E; ++i) {
+      const int e = tid + 256 * i;
+      if (e < H * BS) {
+        const int a = e / BS, b = e % BS;
+        for (int r = 0; r < nx; ++r) {
+          const double w = A[(x0 + r) * H + a];
+          const double2 t = T[r * BS + b];
+          s[i].x = fma(t.x, w, s[i].x);
+          s[i].y = fma(t.y, w, s[i].y);
+        }
+      }
+    }
+  }
+  C* o = out + ((size_t)blockIdx.y * stride + blockIdx.x) * (size_t)(H * H);
+#pragma unroll
+  for (int i = 0; i < E; ++i) {
+    const int e = tid + 256 * i;
+    const int x = e / BS, y = b0 + e % BS;
+    if (e < H * BS) o[x * H + folded_at(2 * H, y)] = from_d<C>(s[i]);
+  }
+}
+
+// Smallest transform length of the kernels that is at least 2 box - 1.  Both the
+// input and the needed output of a propagation lie in the box, so only the
+// offsets |d| < box of the propagator's N x N convolution kernel are ever used:
+// a circular convolution with that kernel truncated to them, of any length >=
+// 2 box - 1, gives the same field (in FP64 to 2e-14 after 100 bounces).  In
+// complex64 the field is closer to it than by the grid's own transform: 3.7e-6
+// against 1.2e-5 after 100 bounces of 10 disks at 128^2 (length 80), since
+// fewer rounded roots act on a mode in each bounce; the spectrum's entries are
+// rounded to nearest (keeping more of their bits changes nothing).
+int compact_length(int box, bool fp64) {
+  // complex128 takes neither 160 (40 points a thread) nor 40 (20 points for 2
+  // threads a line: the one-frequency dancer at 64^2, whose few lines leave an
+  // FP64 instruction's 16 cycles a warp exposed, took 12.0 ms against 7.5 ms at
+  // length 64 with 8 points a thread)
+  for (int M : {8, 16, 32, 40, 64, 80, 128, 160, 256})
+    if (M >= 2 * box - 1 && !(fp64 && (M == 40 || M == 160))) return M;
+  return 0;
+}
+
+// A[q][a] (q over the non-negative wavenumbers of the n-point grid: q + 1/2 for
+// even n, q for odd n, in units of 2 pi / (n dx); a < M/2: the wavenumber
+// (a + 1/2) of the M-point transform): weight (2, or 1 at wavenumber 0) / (n M)
+// times sum_{|d| < box} cos(2 pi q' d / n) cos(2 pi a' d / M).
+std::vector<double> compact_matrix(int n, int M, int box) {
+  const int Q = (n + 1) / 2, H = M / 2;
+  const bool even = n % 2 == 0;
+  // sum_{|d| < box} cos(theta d), theta / 2 = pi num / (2 n M)
+  auto dirichlet = [&](long long num) {
+    const double den = 2.0 * n * M;
+    const double s = sin(M_PI * (double)num / den);
+    if (num % (2LL * n * M) == 0) return 2.0 * box - 1.0;
+    return sin(M_PI * (double)((num * (2LL * box - 1)) % (4LL * n * M)) / den) / s;
+  };
+  std::vector<double> A((size_t)Q * H);
+  for (int q = 0; q < Q; ++q)
+    for (int a = 0; a < H; ++a) {
+      // theta / 2 = pi (q'/n -+ a'/M), 2 q' and 2 a' whole
+      const long long x = (long long)(even ? 2 * q + 1 : 2 * q) * M, y = (long long)(2 * a + 1) * n;
+      const double sum = 0.5 * (dirichlet(x - y) + dirichlet(x + y));
+      A[(size_t)q * H + a] = (!even && q == 0 ? 1.0 : 2.0) / ((double)n * M) * sum;
+    }
+  return A;
+}
+
+int launch_compact_table(bool fp64, void* out, int nfreq, const double* d_freqs, int ntab, int stride,
+                         const int* d_regions, const RegionGeo* d_geo, int n, const double* d_kX, const double* d_kY,
+                         const double* d_A, int M, cudaStream_t st) {
+  if (ntab <= 0 || nfreq <= 0) return 0;
+  const int Q = (n + 1) / 2, H = M / 2, first = n / 2;
+  const int BS = H <= 40 ? H : H == 80 ? 40 : 32;
+  const size_t smem = sizeof(double2) * kChunk * (Q + BS);
+  dim3 grid(ntab, nfreq, H / BS);
+  auto go = [&](auto* o, auto e) {
+    using C = std::remove_pointer_t<decltype(o)>;
+    constexpr int E = decltype(e)::value;
+    const cudaError_t rc = cudaFuncSetAttribute(k_compact_table<C, E>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxSmem);
+    if (rc != cudaSuccess) return (int)rc;
+    COUNT_LAUNCH();
+    k_compact_table<C, E><<<grid, 256, smem, st>>>(o, d_freqs, stride, d_regions, d_geo, Q, first, d_kX, d_kY, d_A, H, BS);
+    return (int)cudaGetLastError();
+  };
+  using std::integral_constant;
+  const int per = H * BS;
+  if (smem > kMaxSmem) return (int)cudaErrorInvalidValue;
+  if (fp64) {
+    double2* o = (double2*)out;
+    return per <= 512 ? go(o, integral_constant<int, 2>()) : per <= 2048 ? go(o, integral_constant<int, 8>())
+                                                                       : go(o, integral_constant<int, 16>());
+  }
+  float2* o = (float2*)out;
+  return per <= 512 ? go(o, integral_constant<int, 2>()) : per <= 2048 ? go(o, integral_constant<int, 8>())
+                                                                     : go(o, integral_constant<int, 16>());
 }
 
 template <typename C>
@@ -1297,7 +790,7 @@ int launch_exit_combine(double2* out, const double2* full, const double2* direct
 }
 
 __global__ void k_embed_box(double2* full, const double2* box, int nfreq, int nx, int ny, int nbx,
-                            int nby, int bx0, int by0) {
+                            int nby, int bx0, int by0, double alpha) {
   const size_t total = (size_t)nfreq * nx * ny;
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
     const int x = (int)(i % nx);
@@ -1305,16 +798,19 @@ __global__ void k_embed_box(double2* full, const double2* box, int nfreq, int nx
     const size_t f = i / ((size_t)nx * ny);
     const int ix = x - bx0, iy = y - by0;
     double2 v = make_double2(0.0, 0.0);
-    if (ix >= 0 && ix < nbx && iy >= 0 && iy < nby) v = box[(f * nby + iy) * nbx + ix];
+    if (ix >= 0 && ix < nbx && iy >= 0 && iy < nby) {
+      v = box[(f * nby + iy) * nbx + ix];
+      if (alpha != 0.0) v = cmul(v, dcexp(0.0, -alpha * (ix + iy)));   // the stages' fields carry exp(i alpha (x + y))
+    }
     full[i] = v;
   }
 }
 
 int launch_embed_box(double2* full, const double2* box, int nfreq, int nx, int ny, int nbx, int nby,
-                     int bx0, int by0, cudaStream_t st) {
+                     int bx0, int by0, double alpha, cudaStream_t st) {
   size_t total = (size_t)nfreq * nx * ny;
   COUNT_LAUNCH();
-  k_embed_box<<<grid1d(total), 256, 0, st>>>(full, box, nfreq, nx, ny, nbx, nby, bx0, by0);
+  k_embed_box<<<grid1d(total), 256, 0, st>>>(full, box, nfreq, nx, ny, nbx, nby, bx0, by0, alpha);
   return (int)cudaGetLastError();
 }
 

@@ -32,15 +32,16 @@ struct FusedArgs {
   int nfreq;          // frequencies in the batch (grid.y)
   int nbx, nby;       // pruned box (pixels that the disk mask can reach)
   int nslots;         // state slots per frequency
-  int ntab;           // regions per frequency in the phasor table
+  int ntab;           // tables per frequency that the phasor buffer has room for
   int fold;           // phasor table stores one quadrant (N/2 x N/2)
   C* state;           // [f][slot][nby][nbx]
-  const C* phasor;    // [f][region][N/2][N/2] (fold) or [f][region][N][N], 1/N^2 included
+  const C* phasor;    // [f][table][N/2][N/2] (fold) or [f][table][N][N], 1/N^2 included
+  const int* tab_idx; // [region] -> table (regions of equal thickness and permittivity share one)
   const C* tilt;      // [f][tilt_idx][nby][nbx]
   const int* tilt_idx;            // [region] -> tilt map index, -1 = identity
   int ntilt;                      // tilt maps per frequency
   const unsigned char* mask;      // [nby][nbx]
-  const double2* coefs;           // [coef][4]
+  const C* coefs;                 // [coef][4]
   double2* exitacc;               // [exit][f][nby][nbx]
   const C* addbuf;                // [add][nby][nbx] (frequency independent)
   const StepDesc* steps;          // this stage
@@ -66,8 +67,9 @@ enum FusedVariant {
 // The variants valid for a stage of this shape (kFusedRule first).
 std::vector<int> fused_variants(int N, int nbx, int nby, bool fp64);
 
-// Launch the fused stage kernel (templated on the grid size N and the field
-// precision).  Returns a cudaError_t.
+// Launch the fused stage kernel (templated on the transform length N and the
+// field precision).  N is the grid's size, or compact_length(box).  Returns a
+// cudaError_t.
 int launch_fused_stage_f(int N, const FusedArgs<float2>& a, int nsteps, cudaStream_t st);
 int launch_fused_stage_d(int N, const FusedArgs<double2>& a, int nsteps, cudaStream_t st);
 size_t fused_smem_bytes(int N, int nbx, int nby, bool fp64);
@@ -79,6 +81,14 @@ bool fused_supported(int N, int nbx, int nby, bool fp64);
 // tiles it needs for a stage of nsteps steps, and whether a stage takes it.
 size_t split_tile_bytes(int N, int nby, int nfreq, int nsteps, bool fp64);
 bool split_stage(int nsteps, int nfreq);
+bool split_length(int N);
+
+// Shortest transform length of the fused kernel that gives the fields of a box
+// of `box` pixels exactly (the propagator's kernel truncated to the offsets
+// within the box), 0 if there is none; the matrix that takes a grid's phasors
+// to that transform's spectrum.
+int compact_length(int box, bool fp64);
+std::vector<double> compact_matrix(int n, int M, int box);
 
 // ---- split-TF32 tensor-core GEMM (bf_tcgemm.cu) --------------------------
 // out[z][n][m] (FP32) = sum over the z-th of `splits` K slices of
@@ -103,10 +113,16 @@ struct RegionGeo {
   double eps_re, eps_im;
   double tilt_x, tilt_y;
 };
-// phasor[f][t][..] for table regions t (region ids in regions[t]); 1/(N*N) folded in.
-int launch_phasor_table(bool fp64, void* out, int nfreq, const double* d_freqs, int ntab,
+// phasor[f][t][..] for the ntab tables t (region ids in regions[t]), `stride`
+// tables apart per frequency; 1/(N*N) folded in.
+int launch_phasor_table(bool fp64, void* out, int nfreq, const double* d_freqs, int ntab, int stride,
                         const int* d_regions, const RegionGeo* d_geo, int N, const double* d_kX,
                         const double* d_kY, int fold, cudaStream_t st);
+// The same for a compact transform of length M on an n x n grid (always one
+// quadrant, M/2 x M/2); d_A = compact_matrix(n, M, box).
+int launch_compact_table(bool fp64, void* out, int nfreq, const double* d_freqs, int ntab, int stride,
+                         const int* d_regions, const RegionGeo* d_geo, int n, const double* d_kX, const double* d_kY,
+                         const double* d_A, int M, cudaStream_t st);
 // tilt[f][m][nby][nbx] = exp(-i k0 (tx x + ty y)) * exp(-i k0 surf) for map m of region regions[m]
 int launch_tilt_table(bool fp64, void* out, int nfreq, const double* d_freqs, int nmaps,
                       const int* d_regions, const RegionGeo* d_geo, int nbx, int nby, int bx0,
@@ -139,9 +155,10 @@ int launch_convert(const void* in, bool in_fp64, void* out, bool out_fp64, size_
 // out[f][ny][nx] (complex128) = direct[ny][nx] + coef * full[f][ny][nx]
 int launch_exit_combine(double2* out, const double2* full, const double2* direct,
                         double2 coef, int nfreq, int npix, cudaStream_t st);
-// embed box acc [f][nby][nbx] (FP64) into full grid [f][ny][nx] (FP64)
+// embed box acc [f][nby][nbx] (FP64) times exp(-i alpha (x + y)), x and y from
+// the box's corner, into full grid [f][ny][nx] (FP64)
 int launch_embed_box(double2* full, const double2* box, int nfreq, int nx, int ny, int nbx,
-                     int nby, int bx0, int by0, cudaStream_t st);
+                     int nby, int bx0, int by0, double alpha, cudaStream_t st);
 // state[f][slot][..] = init[slot][..] converted, for all f
 int launch_broadcast_state(bool fp64, void* state, const double2* init, int nfreq,
                            size_t per_freq, cudaStream_t st);
@@ -170,6 +187,14 @@ struct Rfp1dArgs {
 int launch_rfp1d(bool fp64, const Rfp1dArgs& a, cudaStream_t st);
 
 void init_constant_roots();  // host: fill the unit-root tables (once per device)
+void fill_roots(int n, double2* hd, float2* hf);   // exp(-2 pi i k / n), k < n, n a multiple of 8
+// bf_five_f.cu / bf_five_d.cu: their unit-root tables, stage launches and variants
+void init_roots_five_f();
+void init_roots_five_d();
+int launch_five_f(int N, const FusedArgs<float2>& a, int nsteps, cudaStream_t st);
+int launch_five_d(int N, const FusedArgs<double2>& a, int nsteps, cudaStream_t st);
+std::vector<int> five_variants_f(int N, int nby);
+std::vector<int> five_variants_d(int N, int nby);
 
 // Kernel launches issued by this library since load (for launch accounting).
 unsigned long long launch_count();

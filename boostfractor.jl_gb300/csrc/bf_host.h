@@ -108,10 +108,12 @@ struct StageGraph {
 // steady-state path) and the cached bounce plan.
 struct Workspace {
   DBuf freq, reg, phasor, tidx, tregs, tilt, init, state, add, coef, exitacc, steps, tmp, beta, mg;
+  DBuf tab_idx, compact_A;       // table of each region; compact_matrix
   DBuf exit_full[2], direct[2];
   std::string plan_key;  // solver/nmax/emission of the cached plan
   std::vector<size_t> stage_off, stage_len;
   int nslots = 0, ntab = 0, ntilt = 0, nexit = 0, nadd = 0;
+  std::vector<int> tab_region;   // region of each of the plan's ntab table indices
   std::vector<int> exit_region;
   std::vector<std::complex<double>> exit_coef;
   std::vector<int> has_direct;
