@@ -956,31 +956,64 @@ struct ChainRegion {
   double2 S;             // axion S factor of the step
 };
 
+// 16 or 8 bytes from global to shared memory, asynchronously
+__device__ __forceinline__ void chain_copy(double2* dst, const double2* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
+}
+
+// FP64 chain.  Row r of T21 and T22 (and entry r of the axion beam) depends on
+// row r only, so a frequency's rows spread over gridDim.y CTAs of `rows` rows
+// each, with nothing to exchange.  Bound by the FP64 pipe: 28 modes at 29
+// frequencies took 4.29 ms with a CTA per frequency (29 of 152 SMs busy, T in
+// global memory), 0.86 ms here.
 template <typename C>
-__global__ void __launch_bounds__(256) k_chain(const C* P, const C* Pinv, const ChainRegion* cr, int nd,
-                                               int nm, const double2* emit, C* T21g, C* T22g,
-                                               double2* axg) {
+__global__ void __launch_bounds__(512) k_chain(const C* P, const C* Pinv, const ChainRegion* cr, int nd,
+                                               int nm, int rows, int staged, const double2* emit, C* T21g,
+                                               C* T22g, double2* axg) {
   extern __shared__ __align__(16) unsigned char sm[];
-  C* U = reinterpret_cast<C*>(sm);
-  C* V = U + nm * nm;
-  double2* ax = reinterpret_cast<double2*>(V + nm * nm);
-  double2* em = ax + nm;
   const int f = blockIdx.x, tid = threadIdx.x, nt = blockDim.x;
-  C* T21 = T21g + (size_t)f * nm * nm;
-  C* T22 = T22g + (size_t)f * nm * nm;
-  for (int e = tid; e < nm * nm; e += nt) {
+  const int r0 = blockIdx.y * rows, nr = min(rows, nm - r0), ne = nr * nm;
+  C* U = reinterpret_cast<C*>(sm);
+  C* V = U + ne;
+  C* T21 = V + ne;
+  C* T22 = T21 + ne;
+  double2* ax = reinterpret_cast<double2*>(T22 + ne);
+  double2* em = ax + nr;
+  // with `staged`: this region's and the next one's P and inverse(P), copied
+  // while the products of the region before run
+  const int n2 = nm * nm;
+  C* stage = reinterpret_cast<C*>(em + nm);
+  auto fetch = [&](int j) {
+    if (staged && j < nd) {
+      const C* Pj = P + ((size_t)f * nd + j) * n2;
+      const C* Qj = Pinv + ((size_t)f * nd + j) * n2;
+      C* d = stage + (j & 1) * 2 * n2;
+      for (int e = tid; e < n2; e += nt) {
+        chain_copy(d + e, Pj + e);
+        chain_copy(d + n2 + e, Qj + e);
+      }
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  fetch(1);
+  for (int e = tid; e < ne; e += nt) {
     T21[e] = dto<C>(make_double2(0.0, 0.0));
-    T22[e] = dto<C>(make_double2((e / nm) == (e % nm) ? 1.0 : 0.0, 0.0));
+    T22[e] = dto<C>(make_double2(r0 + (e / nm) == (e % nm) ? 1.0 : 0.0, 0.0));
   }
-  for (int m = tid; m < nm; m += nt) {
-    ax[m] = make_double2(0.0, 0.0);
-    em[m] = emit[m];
-  }
+  for (int m = tid; m < nr; m += nt) ax[m] = make_double2(0.0, 0.0);
+  for (int m = tid; m < nm; m += nt) em[m] = emit[m];
   __syncthreads();
   for (int j = 1; j < nd; ++j) {
     const ChainRegion g = cr[j];
+    // U = a T21 + b T22, V = b T21 + a T22
+    const C a = dto<C>(g.a), b = dto<C>(g.b), s = dto<C>(g.inv2n);
+    for (int e = tid; e < ne; e += nt) {
+      const C t1 = T21[e], t2 = T22[e];
+      U[e] = bf::cadd(bf::cmul(a, t1), bf::cmul(b, t2));
+      V[e] = bf::cadd(bf::cmul(b, t1), bf::cmul(a, t2));
+    }
     // axion_beam += S (T21 + T22) emit   (uses T of the previous step)
-    for (int m = tid; m < nm; m += nt) {
+    for (int m = tid; m < nr; m += nt) {
       double2 acc = make_double2(0.0, 0.0);
       for (int k = 0; k < nm; ++k) {
         const double2 t = bf::to_d(bf::cadd(T21[m * nm + k], T22[m * nm + k]));
@@ -988,34 +1021,34 @@ __global__ void __launch_bounds__(256) k_chain(const C* P, const C* Pinv, const 
       }
       ax[m] = bf::cadd(ax[m], bf::cmul(g.S, acc));
     }
-    // U = a T21 + b T22, V = b T21 + a T22
-    const C a = dto<C>(g.a), b = dto<C>(g.b), s = dto<C>(g.inv2n);
-    for (int e = tid; e < nm * nm; e += nt) {
-      const C t1 = T21[e], t2 = T22[e];
-      U[e] = bf::cadd(bf::cmul(a, t1), bf::cmul(b, t2));
-      V[e] = bf::cadd(bf::cmul(b, t1), bf::cmul(a, t2));
-    }
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
     __syncthreads();
-    const C* Pj = P + (((size_t)f * nd + j) * nm) * nm;
-    const C* Qj = Pinv + (((size_t)f * nd + j) * nm) * nm;
+    fetch(j + 1);
+    const C* Pj = staged ? stage + (j & 1) * 2 * n2 : P + ((size_t)f * nd + j) * n2;
+    const C* Qj = staged ? Pj + n2 : Pinv + ((size_t)f * nd + j) * n2;
     // T21 = s U P, T22 = s V Pinv
-    for (int e = tid; e < nm * nm; e += nt) {
+    for (int e = tid; e < ne; e += nt) {
       const int r = e / nm, c = e % nm;
       C acc1 = dto<C>(make_double2(0.0, 0.0)), acc2 = acc1;
+#pragma unroll 4
       for (int k = 0; k < nm; ++k) {
         const C u = U[r * nm + k], v = V[r * nm + k];
         const C p = Pj[k * nm + c], q = Qj[k * nm + c];
-        acc1.x += u.x * p.x - u.y * p.y;
-        acc1.y += u.x * p.y + u.y * p.x;
-        acc2.x += v.x * q.x - v.y * q.y;
-        acc2.y += v.x * q.y + v.y * q.x;
+        acc1.x = fma(u.x, p.x, fma(-u.y, p.y, acc1.x));
+        acc1.y = fma(u.x, p.y, fma(u.y, p.x, acc1.y));
+        acc2.x = fma(v.x, q.x, fma(-v.y, q.y, acc2.x));
+        acc2.y = fma(v.x, q.y, fma(v.y, q.x, acc2.y));
       }
       T21[e] = bf::cmul(s, acc1);
       T22[e] = bf::cmul(s, acc2);
     }
     __syncthreads();
   }
-  for (int m = tid; m < nm; m += nt) axg[(size_t)f * nm + m] = ax[m];
+  for (int m = tid; m < nr; m += nt) axg[(size_t)f * nm + r0 + m] = ax[m];
+  for (int e = tid; e < ne; e += nt) {
+    T21g[((size_t)f * nm + r0) * nm + e] = T21[e];
+    T22g[((size_t)f * nm + r0) * nm + e] = T22[e];
+  }
 }
 
 // ---- the chain in double-float (mixed path) -----------------------------------
@@ -1090,6 +1123,223 @@ __device__ __forceinline__ DFc dfc_add(DFc x, DFc y) {
   r.il = e + x.il + y.il;
   df_fast_two_sum(r.ih, r.il);
   return r;
+}
+
+// Two double-floats side by side (T21's and T22's), through Blackwell's packed
+// FP32x2 instructions: half the issue slots, every lane rounded like the scalar
+// form.
+__device__ __forceinline__ float2 p2_add(float2 a, float2 b) {
+  float2 d;
+  asm("{\n\t.reg .b64 x, y, z;\n\tmov.b64 x, {%2, %3};\n\tmov.b64 y, {%4, %5};\n\tadd.rn.f32x2 z, x, y;\n\t"
+      "mov.b64 {%0, %1}, z;\n\t}" : "=f"(d.x), "=f"(d.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+  return d;
+}
+__device__ __forceinline__ float2 p2_sub(float2 a, float2 b) {
+  float2 d;
+  asm("{\n\t.reg .b64 x, y, z;\n\tmov.b64 x, {%2, %3};\n\tmov.b64 y, {%4, %5};\n\tsub.rn.f32x2 z, x, y;\n\t"
+      "mov.b64 {%0, %1}, z;\n\t}" : "=f"(d.x), "=f"(d.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+  return d;
+}
+__device__ __forceinline__ float2 p2_mul(float2 a, float2 b) {
+  float2 d;
+  asm("{\n\t.reg .b64 x, y, z;\n\tmov.b64 x, {%2, %3};\n\tmov.b64 y, {%4, %5};\n\tmul.rn.f32x2 z, x, y;\n\t"
+      "mov.b64 {%0, %1}, z;\n\t}" : "=f"(d.x), "=f"(d.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+  return d;
+}
+__device__ __forceinline__ float2 p2_fma(float2 a, float2 b, float2 c) {
+  float2 d;
+  asm("{\n\t.reg .b64 x, y, w, z;\n\tmov.b64 x, {%2, %3};\n\tmov.b64 y, {%4, %5};\n\tmov.b64 w, {%6, %7};\n\t"
+      "fma.rn.f32x2 z, x, y, w;\n\tmov.b64 {%0, %1}, z;\n\t}"
+      : "=f"(d.x), "=f"(d.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
+  return d;
+}
+__device__ __forceinline__ float2 p2_neg(float2 a) { return make_float2(-a.x, -a.y); }
+struct DF2 { float2 rh, rl, ih, il; };
+__device__ __forceinline__ void p2_two_sum(float2 a, float2 b, float2& s, float2& e) {
+  s = p2_add(a, b);
+  const float2 z = p2_sub(s, a);
+  e = p2_add(p2_sub(a, p2_sub(s, z)), p2_sub(b, z));
+}
+__device__ __forceinline__ void p2_fast_two_sum(float2& hi, float2& lo) {
+  const float2 t = p2_add(hi, lo);
+  lo = p2_sub(lo, p2_sub(t, hi));
+  hi = t;
+}
+// (sh, sl) += a b, the product exact; nb = -b gives its rounding error by one FMA
+__device__ __forceinline__ void p2_acc_prod(float2& sh, float2& sl, float2 a, float2 b) {
+  const float2 p = p2_mul(a, b);
+  const float2 e = p2_fma(a, b, p2_neg(p));
+  float2 t, d;
+  p2_two_sum(sh, p, t, d);
+  sh = t;
+  sl = p2_add(sl, p2_add(d, e));
+}
+__device__ __forceinline__ DF2 df2_add(DF2 x, DF2 y) {
+  DF2 r;
+  float2 e;
+  p2_two_sum(x.rh, y.rh, r.rh, e);
+  r.rl = p2_add(p2_add(e, x.rl), y.rl);
+  p2_fast_two_sum(r.rh, r.rl);
+  p2_two_sum(x.ih, y.ih, r.ih, e);
+  r.il = p2_add(p2_add(e, x.il), y.il);
+  p2_fast_two_sum(r.ih, r.il);
+  return r;
+}
+// (h, l) = xh yh + ... for real x: one component of a real times a complex double-float
+__device__ __forceinline__ void p2_mul_df(float2 xh, float2 xl, float2 yh, float2 yl, float2& h, float2& l) {
+  h = p2_mul(xh, yh);
+  l = p2_add(p2_fma(xh, yh, p2_neg(h)), p2_fma(xl, yh, p2_mul(xh, yl)));
+  p2_fast_two_sum(h, l);
+}
+template <bool REAL>
+__device__ __forceinline__ DF2 df2_mul(DF2 x, DF2 y) {
+  DF2 r;
+  if (REAL) {
+    p2_mul_df(x.rh, x.rl, y.rh, y.rl, r.rh, r.rl);
+    p2_mul_df(x.rh, x.rl, y.ih, y.il, r.ih, r.il);
+    return r;
+  }
+  const float2 z = make_float2(0.f, 0.f);
+  float2 sh = z, sl = z;
+  p2_acc_prod(sh, sl, x.rh, y.rh);
+  p2_acc_prod(sh, sl, p2_neg(x.ih), y.ih);
+  sl = p2_add(sl, p2_sub(p2_fma(x.rl, y.rh, p2_mul(x.rh, y.rl)), p2_fma(x.il, y.ih, p2_mul(x.ih, y.il))));
+  p2_fast_two_sum(sh, sl);
+  r.rh = sh;
+  r.rl = sl;
+  sh = sl = z;
+  p2_acc_prod(sh, sl, x.rh, y.ih);
+  p2_acc_prod(sh, sl, x.ih, y.rh);
+  sl = p2_add(sl, p2_add(p2_fma(x.rl, y.ih, p2_mul(x.rh, y.il)), p2_fma(x.il, y.rh, p2_mul(x.ih, y.rl))));
+  p2_fast_two_sum(sh, sl);
+  r.ih = sh;
+  r.il = sl;
+  return r;
+}
+__device__ __forceinline__ float2 p2_shfl(float2 v, int src, int width) {
+  return make_float2(__shfl_sync(0xffffffffu, v.x, src, width), __shfl_sync(0xffffffffu, v.y, src, width));
+}
+__device__ __forceinline__ DFc dfc_shfl_xor(DFc v, int mask, int width) {
+  return {__shfl_xor_sync(0xffffffffu, v.rh, mask, width), __shfl_xor_sync(0xffffffffu, v.rl, mask, width),
+          __shfl_xor_sync(0xffffffffu, v.ih, mask, width), __shfl_xor_sync(0xffffffffu, v.il, mask, width)};
+}
+
+// A region's chain factors in double-float (split on the host: the FP64
+// conversions of a CTA's every warp and region cost more than its products at
+// few modes, at 1/64 of the FP32 rate).
+struct ChainRegionDF {
+  DFc a, b, inv2n;
+  double2 S;
+  int real, pad[3];   // a, b and inv2n real
+};
+
+// The double-float chain for nm <= NM (8 or 16): a warp takes 32 / NM rows of
+// one frequency's T, NM lanes a row, and needs no other warp (rows are
+// independent): entries of T in registers, a row's U and V by shuffles, the
+// region's P and inverse(P) columns in registers, loaded a region ahead.  The
+// axion terms wait in shared memory for one FP64 pass at the end.  The values
+// are k_chain_df's, but for the order of a row's axion sum.  Bound by the issue
+// of the double-float products (about 1000 instructions a warp and region): 8
+// modes, 41 regions took 132 us at 256 frequencies (two barriers and a serial
+// axion sum a region, latency-bound) and 737 us at 4096, 51 and 442 us here.
+constexpr int kSegWarps = 2;
+template <int NM>
+__global__ void __launch_bounds__(32 * kSegWarps) k_chain_df_seg(const float2* P, const float2* Pinv,
+                                                                 const ChainRegionDF* crg, int nd, int nm, int nf, const double2* emit,
+                                                                 double2* axg, double2* T21out, double2* T22out) {
+  extern __shared__ __align__(16) unsigned char sm[];
+  constexpr int RW = 32 / NM;   // rows per warp
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, c = lane % NM, rl = lane / NM;
+  const int wpf = (nm + RW - 1) / RW;   // warps per frequency
+  const int task = blockIdx.x * kSegWarps + warp;
+  DFc* axs = reinterpret_cast<DFc*>(sm) + (size_t)warp * nd * RW;   // [region][row of the warp]
+  // the regions' factors in shared memory: read per region from global memory
+  // they cost a cache miss each, 30 % of a warp's time
+  ChainRegionDF* cr = reinterpret_cast<ChainRegionDF*>(reinterpret_cast<DFc*>(sm) + (size_t)kSegWarps * nd * RW);
+  for (int i = threadIdx.x; i < nd * (int)(sizeof(ChainRegionDF) / sizeof(float4)); i += blockDim.x)
+    reinterpret_cast<float4*>(cr)[i] = reinterpret_cast<const float4*>(crg)[i];
+  __syncthreads();
+  if (task >= nf * wpf) return;   // the whole warp leaves together
+  const int f = task / wpf, row = (task % wpf) * RW + rl;
+  const int n2 = nm * nm;
+  const bool col = c < nm;
+  const float2* pj = P + ((size_t)f * nd + 1) * n2 + c;
+  const float2* qj = Pinv + ((size_t)f * nd + 1) * n2 + c;
+  const float2 z2 = make_float2(0.f, 0.f);
+  float2 pn[NM], qn[NM];
+  auto fetch = [&]() {
+#pragma unroll
+    for (int k = 0; k < NM; ++k) {
+      pn[k] = col && k < nm ? pj[k * nm] : z2;
+      qn[k] = col && k < nm ? qj[k * nm] : z2;
+    }
+  };
+  if (nd > 1) fetch();
+  const DFc zero = {0.f, 0.f, 0.f, 0.f};
+  const DFc em = col ? dfc_from(emit[c]) : zero;
+  DF2 t = {z2, z2, z2, z2};   // (T21, T22) entry (row, c)
+  if (row == c) t.rh.y = 1.f;
+  for (int j = 1; j < nd; ++j) {
+    float2 px[NM], py[NM];   // (P, inverse(P)) entries (k, c), real and imaginary parts
+#pragma unroll
+    for (int k = 0; k < NM; ++k) {
+      px[k] = make_float2(pn[k].x, qn[k].x);
+      py[k] = make_float2(pn[k].y, qn[k].y);
+    }
+    pj += n2;
+    qj += n2;
+    if (j + 1 < nd) fetch();
+    const DFc a = cr[j].a, b = cr[j].b, sc = cr[j].inv2n;
+    const bool real = cr[j].real != 0;
+    // the row's axion term (T21 + T22) emit, T of the previous step
+    const DFc t1 = {t.rh.x, t.rl.x, t.ih.x, t.il.x}, t2 = {t.rh.y, t.rl.y, t.ih.y, t.il.y};
+    DFc w = dfc_mul(dfc_add(t1, t2), em);
+#pragma unroll
+    for (int o = 1; o < NM; o <<= 1) w = dfc_add(w, dfc_shfl_xor(w, o, NM));
+    if (c == 0) axs[j * RW + rl] = w;
+    // (U, V) = (a, b) T21 + (b, a) T22
+    auto two = [](DFc x, DFc y) {
+      return DF2{make_float2(x.rh, y.rh), make_float2(x.rl, y.rl), make_float2(x.ih, y.ih), make_float2(x.il, y.il)};
+    };
+    DF2 uv;
+    if (real) uv = df2_add(df2_mul<true>(two(a, b), two(t1, t1)), df2_mul<true>(two(b, a), two(t2, t2)));
+    else uv = df2_add(df2_mul<false>(two(a, b), two(t1, t1)), df2_mul<false>(two(b, a), two(t2, t2)));
+    // (T21, T22) = s (U P, V inverse(P))
+    float2 rh = z2, rlo = z2, ih = z2, ilo = z2;
+#pragma unroll
+    for (int k = 0; k < NM; ++k) {
+      if (k >= nm) break;
+      const float2 xrh = p2_shfl(uv.rh, k, NM), xrl = p2_shfl(uv.rl, k, NM);
+      const float2 xih = p2_shfl(uv.ih, k, NM), xil = p2_shfl(uv.il, k, NM);
+      p2_acc_prod(rh, rlo, xrh, px[k]);
+      p2_acc_prod(rh, rlo, p2_neg(xih), py[k]);
+      p2_acc_prod(ih, ilo, xrh, py[k]);
+      p2_acc_prod(ih, ilo, xih, px[k]);
+      rlo = p2_fma(xrl, px[k], p2_fma(p2_neg(xil), py[k], rlo));
+      ilo = p2_fma(xrl, py[k], p2_fma(xil, px[k], ilo));
+    }
+    p2_fast_two_sum(rh, rlo);
+    p2_fast_two_sum(ih, ilo);
+    const DF2 acc = {rh, rlo, ih, ilo};
+    t = real ? df2_mul<true>(two(sc, sc), acc) : df2_mul<false>(two(sc, sc), acc);
+  }
+  // axion_beam = sum_j S_j term_j in FP64: the products by all lanes, then the
+  // sums in region order
+  __syncwarp();
+  for (int e = RW + lane; e < nd * RW; e += 32) {
+    const double2 t = bf::cmul(cr[e / RW].S, dfc_to_d(axs[e]));
+    reinterpret_cast<double2*>(axs)[e] = t;
+  }
+  __syncwarp();
+  if (lane < RW && (task % wpf) * RW + lane < nm) {
+    double2 ax = make_double2(0.0, 0.0);
+    for (int j = 1; j < nd; ++j) ax = bf::cadd(ax, reinterpret_cast<double2*>(axs)[j * RW + lane]);
+    axg[(size_t)f * nm + (task % wpf) * RW + lane] = ax;
+  }
+  if (col && row < nm) {
+    T21out[(size_t)f * n2 + row * nm + c] = dfc_to_d({t.rh.x, t.rl.x, t.ih.x, t.il.x});
+    T22out[(size_t)f * n2 + row * nm + c] = dfc_to_d({t.rh.y, t.rl.y, t.ih.y, t.il.y});
+  }
 }
 
 __global__ void __launch_bounds__(1024) k_chain_df(const float2* P, const float2* Pinv, const ChainRegion* cr,
@@ -1387,111 +1637,98 @@ __global__ void __launch_bounds__(256) k_final_solve(const C* T21g, const C* T22
   }
 }
 
-// The boundary solve of k_final_solve for nm <= NM (8 or 16), one segment of
+// The boundary solve of k_final_solve for nm <= NM (8, 16 or 32), one segment of
 // NM lanes per frequency (32 / NM frequencies per warp): lane r holds row r of
-// [T22 | axion_beam | T21 reflect] in registers, the pivot search is a shuffle
-// argmax (largest |a|^2, lowest row on ties), the pivot row is broadcast by
-// shuffles.  Every entry goes through the operations of k_final_solve in the
-// same order (LU with partial pivoting, then back substitution); only the
-// CTA-wide reductions and barriers are gone.
+// [T22 | axion_beam | T21 reflect] in registers and the pivot search is a
+// shuffle argmax (largest |a|^2, lowest row on ties) over the rows not yet
+// used; rows stay where they are (the pivot's lane is remembered instead of
+// swapping).  A column takes one FP64 division (the pivot's reciprocal), each
+// right-hand side is updated as soon as an unknown is known, and without
+// `reflect` the second one is not solved.  A warp per CTA: its FP64 operations
+// (16 cycles each an SM) run beside no other warp's until every SM has one.
+// 8 modes, 256 frequencies: 112 us with 8 warps a CTA (8 CTAs) and divisions
+// per entry, 20 us; 28 modes at 29 frequencies: 228 us in k_final_solve,
+// 149 us here.
 template <int NM>
-__global__ void __launch_bounds__(256) k_final_solve_warp(const double2* T21g, const double2* T22g,
-                                                          const double2* axg, const double2* reflect, int nm,
-                                                          double2* boost, double2* refl, double* beta2, int* sing,
-                                                          int nf) {
+__global__ void __launch_bounds__(32) k_final_solve_warp(const double2* T21g, const double2* T22g,
+                                                         const double2* axg, const double2* reflect, int nm,
+                                                         double2* boost, double2* refl, double* beta2, int* sing,
+                                                         int nf) {
   constexpr unsigned FULL = 0xffffffffu;
-  constexpr int W = NM + 2, SEG = 32 / NM;
+  constexpr int SEG = 32 / NM;
   const int lane = threadIdx.x & 31, sl = lane % NM;
-  const int first = (blockIdx.x * 8 + (threadIdx.x >> 5)) * SEG;
-  if (first >= nf) return;   // the whole warp leaves together
+  const int first = blockIdx.x * SEG;
   const int fi = first + lane / NM;
   const bool valid = fi < nf;
   const int f = valid ? fi : first;
   const double2* T21 = T21g + (size_t)f * nm * nm;
   const double2* T22 = T22g + (size_t)f * nm * nm;
   const bool row = sl < nm;
-  double2 a[W];
+  double2 a[NM], b0 = make_double2(0.0, 0.0), b1 = b0;
 #pragma unroll
-  for (int k = 0; k < W; ++k) a[k] = make_double2(0.0, 0.0);
+  for (int k = 0; k < NM; ++k) a[k] = row && k < nm ? T22[sl * nm + k] : make_double2(0.0, 0.0);
   if (row) {
-#pragma unroll
-    for (int k = 0; k < NM; ++k)
-      if (k < nm) a[k] = T22[sl * nm + k];
-    a[NM] = axg[(size_t)f * nm + sl];
-    double2 acc = make_double2(0.0, 0.0);
+    b0 = axg[(size_t)f * nm + sl];
     if (reflect)
-      for (int k = 0; k < nm; ++k) acc = bf::cadd(acc, bf::cmul(T21[sl * nm + k], reflect[k]));
-    a[NM + 1] = acc;
+      for (int k = 0; k < nm; ++k) b1 = bf::cadd(b1, bf::cmul(T21[sl * nm + k], reflect[k]));
   }
   auto bcast = [&](double2 v, int src) {
     return make_double2(__shfl_sync(FULL, v.x, src, NM), __shfl_sync(FULL, v.y, src, NM));
   };
+  // a -= x y
+  auto msub = [](double2& z, double2 x, double2 y) {
+    z.x = fma(-x.x, y.x, fma(x.y, y.y, z.x));
+    z.y = fma(-x.x, y.y, fma(-x.y, y.x, z.y));
+  };
+  bool used = false;
+  int my = -1;                 // the column this lane's row is the pivot row of
+  double2 rp = b0;             // and that pivot's reciprocal
 #pragma unroll
   for (int c = 0; c < NM; ++c) {
     if (c >= nm) break;
-    double v = (row && sl >= c) ? a[c].x * a[c].x + a[c].y * a[c].y : -1.0;
-    int p = (row && sl >= c) ? sl : NM;
+    double v = row && !used ? fma(a[c].x, a[c].x, a[c].y * a[c].y) : -1.0;
+    int p = sl;
 #pragma unroll
     for (int o = NM / 2; o > 0; o >>= 1) {
       const double vo = __shfl_xor_sync(FULL, v, o, NM);
       const int po = __shfl_xor_sync(FULL, p, o, NM);
-      if (vo > v || (vo == v && po < p)) { v = vo; p = po; }
+      if (vo > v || (vo == v && po < p) || (vo >= 0.0 && v != v)) { v = vo; p = po; }
     }
-    if (p >= nm) p = c;
-    // swap rows c and p
-    const int src = sl == c ? p : (sl == p ? c : sl);
-#pragma unroll
-    for (int k = 0; k < W; ++k) a[k] = bcast(a[k], src);
-    const double2 piv = bcast(a[c], c);
+    p = __shfl_sync(FULL, p, 0, NM);   // one pivot for the segment, whatever a NaN did to the search
+    const double2 piv = bcast(a[c], p);
     if (valid && sl == 0 && piv.x == 0.0 && piv.y == 0.0) atomicMin(sing, f);   // T22 exactly singular
-    const double d = piv.x * piv.x + piv.y * piv.y;
-    const double2 l = a[c];
-    const double2 fac = make_double2((l.x * piv.x + l.y * piv.y) / d, (l.y * piv.x - l.x * piv.y) / d);
-#pragma unroll
-    for (int k = 0; k < W; ++k) {
-      if (k <= c || (k >= nm && k < NM)) continue;
-      const double2 pk = bcast(a[k], c);
-      if (row && sl > c) a[k] = bf::csub(a[k], bf::cmul(fac, pk));
+    const double id = 1.0 / fma(piv.x, piv.x, piv.y * piv.y);
+    const double2 r = make_double2(piv.x * id, -piv.y * id);
+    if (sl == p) {
+      used = true;
+      my = c;
+      rp = r;
     }
-    if (row && sl > c) a[c] = make_double2(0.0, 0.0);
-  }
-  // back substitution for both right-hand sides, rows nm-1 .. 0
-  double2 x0[NM], x1[NM];
+    const double2 fac = used ? make_double2(0.0, 0.0) : bf::cmul(a[c], r);
 #pragma unroll
-  for (int r = NM - 1; r >= 0; --r) {
-    if (r >= nm) {
-      x0[r] = x1[r] = make_double2(0.0, 0.0);
-      continue;
+    for (int k = c + 1; k < NM; ++k)
+      if (k < nm) msub(a[k], fac, bcast(a[k], p));
+    msub(b0, fac, bcast(b0, p));
+    if (reflect) msub(b1, fac, bcast(b1, p));
+  }
+  // back substitution: unknown c from the row whose pivot it was
+  double s = 0.0;
+#pragma unroll
+  for (int c = NM - 1; c >= 0; --c) {
+    if (c >= nm) continue;
+    const unsigned who = __ballot_sync(FULL, my == c) >> (lane / NM * NM) & (NM == 32 ? FULL : (1u << (NM % 32)) - 1u);
+    const int p = who ? __ffs((int)who) - 1 : 0;
+    const double2 x0 = bcast(bf::cmul(b0, rp), p);
+    if (my != c) msub(b0, x0, a[c]);
+    if (valid && sl == 0) boost[(size_t)f * nm + c] = make_double2(-x0.x, -x0.y);
+    s = fma(x0.x, x0.x, fma(x0.y, x0.y, s));
+    if (reflect) {
+      const double2 x1 = bcast(bf::cmul(b1, rp), p);
+      if (my != c) msub(b1, x1, a[c]);
+      if (valid && sl == 0 && refl) refl[(size_t)f * nm + c] = make_double2(-x1.x, -x1.y);
     }
-    double2 acc0 = a[NM], acc1 = a[NM + 1];
-#pragma unroll
-    for (int k = r + 1; k < NM; ++k) {
-      if (k >= nm) break;
-      acc0 = bf::csub(acc0, bf::cmul(a[k], x0[k]));
-      acc1 = bf::csub(acc1, bf::cmul(a[k], x1[k]));
-    }
-    const double2 pv = a[r];
-    const double dd = pv.x * pv.x + pv.y * pv.y;
-    const double2 s0 = make_double2((acc0.x * pv.x + acc0.y * pv.y) / dd, (acc0.y * pv.x - acc0.x * pv.y) / dd);
-    const double2 s1 = make_double2((acc1.x * pv.x + acc1.y * pv.y) / dd, (acc1.y * pv.x - acc1.x * pv.y) / dd);
-    x0[r] = bcast(s0, r);
-    x1[r] = bcast(s1, r);
   }
-  if (valid && row) {
-#pragma unroll
-    for (int m = 0; m < NM; ++m)
-      if (m == sl) {
-        boost[(size_t)f * nm + m] = make_double2(-x0[m].x, -x0[m].y);
-        if (refl) refl[(size_t)f * nm + m] = make_double2(-x1[m].x, -x1[m].y);
-      }
-  }
-  if (valid && sl == 0 && beta2) {
-    double s = 0.0;
-#pragma unroll
-    for (int m = 0; m < NM; ++m)
-      if (m < nm) s += x0[m].x * x0[m].x + x0[m].y * x0[m].y;
-    beta2[f] = s;
-  }
+  if (valid && sl == 0 && beta2) beta2[f] = s;
 }
 
 // axion_induced_modes / field2modes: c_m = sum conj(Psi_m) B_hat
@@ -2607,12 +2844,57 @@ static int tf_run_t(bf_handle* h, bf_stack* s, bf_modes* md, int nf, const doubl
   TCKS(T22.alloc(h, sizeof(double2) * (size_t)nf * nm * nm));
   TCKS(ax.alloc(h, sizeof(double2) * (size_t)nf * nm));
   if constexpr (fp64) {
-    const size_t smem = sizeof(D2) * 2 * nm * nm + sizeof(double2) * 2 * nm;
+    // rows per CTA: as many CTAs as SMs when the frequencies alone leave SMs
+    // idle, about 256 entries a CTA otherwise
+    const int blocks = std::max(1, std::min(nm, 152 / nf));
+    const int rows = std::max(1, std::min((nm + blocks - 1) / blocks, (256 + nm - 1) / nm));
+    size_t smem = sizeof(D2) * 4 * rows * nm + sizeof(double2) * (rows + nm);
+    const size_t stage = sizeof(D2) * 4 * nm * nm;
+    // matrices staged only while there is about one CTA an SM: more of them hide
+    // the loads, and want the shared memory
+    const int staged = (long long)nf * ((nm + rows - 1) / rows) < 2 * 152 && smem + stage <= 200 * 1024;
+    if (staged) smem += stage;
+    const int threads = std::min(512, (rows * nm + 31) / 32 * 32);
     TCK(cudaFuncSetAttribute(k_chain<D2>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxDynSmem));
     bf::note_launch();
-    k_chain<D2><<<nf, 256, smem, st>>>(Pd, Pinv.as<D2>(), d_cr.as<ChainRegion>(), nd, nm, d_em.as<double2>(),
-                                       T21.as<D2>(), T22.as<D2>(), ax.as<double2>());
+    k_chain<D2><<<dim3(nf, (nm + rows - 1) / rows), threads, smem, st>>>(
+        Pd, Pinv.as<D2>(), d_cr.as<ChainRegion>(), nd, nm, rows, staged, d_em.as<double2>(), T21.as<D2>(), T22.as<D2>(),
+        ax.as<double2>());
     TCK(cudaGetLastError());
+  } else if (nm <= 16 && nd <= 512) {
+    std::vector<ChainRegionDF> crd(nd);
+    static_assert(sizeof(ChainRegionDF) % sizeof(float4) == 0, "copied by 16 bytes");
+    auto split = [](double2 v) {
+      DFc r;
+      r.rh = (float)v.x;
+      r.rl = (float)(v.x - (double)r.rh);
+      r.ih = (float)v.y;
+      r.il = (float)(v.y - (double)r.ih);
+      return r;
+    };
+    for (int j = 1; j < nd; ++j) {
+      crd[j].a = split(cr[j].a);
+      crd[j].b = split(cr[j].b);
+      crd[j].inv2n = split(cr[j].inv2n);
+      crd[j].S = cr[j].S;
+      crd[j].real = cr[j].a.y == 0.0 && cr[j].b.y == 0.0 && cr[j].inv2n.y == 0.0;
+    }
+    DBuf d_crd;
+    TCKS(d_crd.alloc(h, sizeof(ChainRegionDF) * nd));
+    TCK(cudaMemcpyAsync(d_crd.p, crd.data(), sizeof(ChainRegionDF) * nd, cudaMemcpyHostToDevice, st));
+    auto run = [&](auto NMc) -> int {
+      constexpr int NM = decltype(NMc)::value, RW = 32 / NM;
+      const int tasks = nf * ((nm + RW - 1) / RW);
+      const size_t smem = (sizeof(DFc) * kSegWarps * RW + sizeof(ChainRegionDF)) * nd;
+      TCK(cudaFuncSetAttribute(k_chain_df_seg<NM>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxDynSmem));
+      bf::note_launch();
+      k_chain_df_seg<NM><<<(tasks + kSegWarps - 1) / kSegWarps, 32 * kSegWarps, smem, st>>>(
+          Pd, Pinv.as<D2>(), d_crd.as<ChainRegionDF>(), nd, nm, nf, d_em.as<double2>(), ax.as<double2>(),
+          T21.as<double2>(), T22.as<double2>());
+      TCK(cudaGetLastError());
+      return BF_OK;
+    };
+    TCKS(nm <= 8 ? run(std::integral_constant<int, 8>()) : run(std::integral_constant<int, 16>()));
   } else {
     DBuf T21df, T22df, Wdf;
     size_t smem = (sizeof(DFc) * 2 + sizeof(float2) * 2) * nm * nm + (sizeof(double2) + sizeof(DFc)) * nm;
@@ -2647,19 +2929,19 @@ static int tf_run_t(bf_handle* h, bf_stack* s, bf_modes* md, int nf, const doubl
   TCKS(boost.alloc(h, sizeof(cd) * (size_t)nf * nm));
   if (reflect) TCKS(refl.alloc(h, sizeof(cd) * (size_t)nf * nm));
   TCKS(b2.alloc(h, sizeof(double) * nf));
-  if (nm <= 16) {
-    bf::note_launch();
-    if (nm <= 8)
-      k_final_solve_warp<8><<<(nf + 31) / 32, 256, 0, st>>>(T21.as<double2>(), T22.as<double2>(), ax.as<double2>(),
-                                                          reflect ? d_refl.as<double2>() : nullptr, nm,
-                                                          boost.as<double2>(), reflect ? refl.as<double2>() : nullptr,
-                                                          b2.as<double>(), d_sing + 1, nf);
-    else
-      k_final_solve_warp<16><<<(nf + 15) / 16, 256, 0, st>>>(T21.as<double2>(), T22.as<double2>(), ax.as<double2>(),
-                                                           reflect ? d_refl.as<double2>() : nullptr, nm,
-                                                           boost.as<double2>(), reflect ? refl.as<double2>() : nullptr,
-                                                           b2.as<double>(), d_sing + 1, nf);
-    TCK(cudaGetLastError());
+  if (nm <= 32) {
+    auto run = [&](auto NMc) -> int {
+      constexpr int NM = decltype(NMc)::value, SEG = 32 / NM;
+      bf::note_launch();
+      k_final_solve_warp<NM><<<(nf + SEG - 1) / SEG, 32, 0, st>>>(
+          T21.as<double2>(), T22.as<double2>(), ax.as<double2>(), reflect ? d_refl.as<double2>() : nullptr, nm,
+          boost.as<double2>(), reflect ? refl.as<double2>() : nullptr, b2.as<double>(), d_sing + 1, nf);
+      TCK(cudaGetLastError());
+      return BF_OK;
+    };
+    TCKS(nm <= 8    ? run(std::integral_constant<int, 8>())
+         : nm <= 16 ? run(std::integral_constant<int, 16>())
+                    : run(std::integral_constant<int, 32>()));
   } else {
     const size_t smem = sizeof(double2) * nm * (nm + 2) + 256 * (sizeof(double) + sizeof(int));
     TCK(cudaFuncSetAttribute(k_final_solve<double2>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxDynSmem));
