@@ -1228,8 +1228,8 @@ __device__ __forceinline__ DFc dfc_shfl_xor(DFc v, int mask, int width) {
 // conversions of a CTA's every warp and region cost more than its products at
 // few modes, at 1/64 of the FP32 rate).
 struct ChainRegionDF {
-  DFc a, b, inv2n;
-  double2 S;
+  DFc a, b, inv2n, Sd;
+  double2 S;          // Sd in FP64
   int real, pad[3];   // a, b and inv2n real
 };
 
@@ -1345,7 +1345,8 @@ __global__ void __launch_bounds__(32 * kSegWarps) k_chain_df_seg(const float2* P
 __global__ void __launch_bounds__(1024) k_chain_df(const float2* P, const float2* Pinv, const ChainRegion* cr,
                                                   int nd, int nm, const double2* emit, DFc* T21g, DFc* T22g,
                                                   double2* axg, double2* T21out, double2* T22out, int par_axion,
-                                                  DFc* Wg) {
+                                                  DFc* Wg, const int* only) {
+  if (only && !only[blockIdx.x]) return;   // solved by refinement
   extern __shared__ __align__(16) unsigned char sm[];
   const int n2 = nm * nm;
   DFc* U = reinterpret_cast<DFc*>(sm);
@@ -1466,6 +1467,256 @@ __global__ void __launch_bounds__(1024) k_chain_df(const float2* P, const float2
   }
 }
 
+// ---- the boundary solve by refinement (mixed path, 17 to 64 modes) -------------
+// boost solves T22 x + axion_beam = 0 (and refl T22 y + T21 reflect = 0) with
+// T = prod_j G_j blockdiag(P_j, inverse(P_j)).  Only the residual has to be
+// exact, and it needs no T: the bottom half of the regions' action on the
+// vector (reflect or 0, x) plus the axion terms is T21 u + T22 x + axion_beam,
+// two matrix-vector products a region.  So
+//   * k_chain_f32 forms T in complex64 (its error, amplified by cond(T22),
+//     is ~1e-3 of x);
+//   * k_invert_reg inverts T22 in complex64: the correction's approximate inverse;
+//   * k_refine evaluates residuals in double-float (the arithmetic of
+//     k_chain_df, on vectors) and corrects x until the next correction would be
+//     below 1e-9 |x|, 3 to 4 residuals;
+//   * frequencies that do not converge (an ill-conditioned T22, a NaN) are
+//     marked and solved as before (k_chain_df and the FP64 LU).
+// 64 modes, 41 regions, 1024 frequencies: chain and boundary solve 38.5 + 3.3 ms
+// with T in double-float; 6.5 ms here (chain 4.1, 85 GFMA at 0.55 of the FP32
+// rate, inverse 0.2, residuals 2.2).
+template <int NB>
+__global__ void __launch_bounds__((NB / 2) * (NB / 4), NB == 64 ? 1 : 4)
+    k_chain_f32(const float2* P, const float2* Pinv, const ChainRegionDF* cr, int nd, int nm, float2* T22out) {
+  constexpr int NT = (NB / 2) * (NB / 4), CG = NB / 4, UP = NB + 2;
+  extern __shared__ __align__(16) unsigned char sm[];
+  float2* M = reinterpret_cast<float2*>(sm);            // [2][P, inverse(P)][NB][NB]
+  float2* Us = M + 4 * NB * NB;                         // [k][row], pitch UP
+  float2* Vs = Us + NB * UP;
+  const int tid = threadIdx.x, f = blockIdx.x;
+  // rows r0, r0 + 1; columns c0, c0 + 1, c0 + NB / 2, c0 + NB / 2 + 1
+  const int r0 = 2 * (tid / CG), c0 = 2 * (tid % CG);
+  const int n2 = nm * nm;
+  auto col = [&](int i) { return c0 + (i & 1) + (i >> 1) * (NB / 2); };
+  auto fetch = [&](int j) {
+    if (j < nd) {
+      const float2* src[2] = {P + ((size_t)f * nd + j) * n2, Pinv + ((size_t)f * nd + j) * n2};
+      for (int w = 0; w < 2; ++w) {
+        float2* d = M + ((j & 1) * 2 + w) * NB * NB;
+        for (int e = tid; e < n2; e += NT)
+          asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(
+                           (unsigned)__cvta_generic_to_shared(d + (nm == NB ? e : e / nm * NB + e % nm))),
+                       "l"(src[w] + e)
+                       : "memory");
+      }
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  // entries beyond nm stay zero
+  if (nm < NB)
+    for (int e = tid; e < 4 * NB * NB; e += NT) M[e] = make_float2(0.f, 0.f);
+  __syncthreads();
+  fetch(1);
+  float2 t1[2][4], t2[2][4];
+#pragma unroll
+  for (int r = 0; r < 2; ++r)
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      t1[r][i] = make_float2(0.f, 0.f);
+      t2[r][i] = make_float2(r0 + r == col(i) ? 1.f : 0.f, 0.f);
+    }
+  for (int j = 1; j < nd; ++j) {
+    const DFc ad = cr[j].a, bd = cr[j].b, sd = cr[j].inv2n;
+    // the region's factors with 1 / (2 n) folded in
+    const float2 s = make_float2(sd.rh, sd.ih);
+    const float2 a = bf::cmul(make_float2(ad.rh, ad.ih), s), b = bf::cmul(make_float2(bd.rh, bd.ih), s);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      float2 u[2], v[2];
+#pragma unroll
+      for (int r = 0; r < 2; ++r) {
+        u[r] = bf::cadd(bf::cmul(a, t1[r][i]), bf::cmul(b, t2[r][i]));
+        v[r] = bf::cadd(bf::cmul(b, t1[r][i]), bf::cmul(a, t2[r][i]));
+      }
+      *reinterpret_cast<float4*>(Us + col(i) * UP + r0) = make_float4(u[0].x, u[0].y, u[1].x, u[1].y);
+      *reinterpret_cast<float4*>(Vs + col(i) * UP + r0) = make_float4(v[0].x, v[0].y, v[1].x, v[1].y);
+    }
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncthreads();
+    fetch(j + 1);
+    const float2* Pj = M + (j & 1) * 2 * NB * NB;
+    const float2* Qj = Pj + NB * NB;
+#pragma unroll
+    for (int r = 0; r < 2; ++r)
+#pragma unroll
+      for (int i = 0; i < 4; ++i) t1[r][i] = t2[r][i] = make_float2(0.f, 0.f);
+    auto mac = [](float2& z, float2 x, float2 y) {
+      z.x = fmaf(x.x, y.x, fmaf(-x.y, y.y, z.x));
+      z.y = fmaf(x.x, y.y, fmaf(x.y, y.x, z.y));
+    };
+#pragma unroll 2
+    for (int k = 0; k < nm; ++k) {
+      const float4 u = *reinterpret_cast<const float4*>(Us + k * UP + r0);
+      const float4 v = *reinterpret_cast<const float4*>(Vs + k * UP + r0);
+      float4 p[2], q[2];
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        p[h] = *reinterpret_cast<const float4*>(Pj + k * NB + c0 + h * (NB / 2));
+        q[h] = *reinterpret_cast<const float4*>(Qj + k * NB + c0 + h * (NB / 2));
+      }
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const float2 p0 = make_float2(p[h].x, p[h].y), p1 = make_float2(p[h].z, p[h].w);
+        const float2 q0 = make_float2(q[h].x, q[h].y), q1 = make_float2(q[h].z, q[h].w);
+        mac(t1[0][2 * h], make_float2(u.x, u.y), p0);
+        mac(t1[0][2 * h + 1], make_float2(u.x, u.y), p1);
+        mac(t1[1][2 * h], make_float2(u.z, u.w), p0);
+        mac(t1[1][2 * h + 1], make_float2(u.z, u.w), p1);
+        mac(t2[0][2 * h], make_float2(v.x, v.y), q0);
+        mac(t2[0][2 * h + 1], make_float2(v.x, v.y), q1);
+        mac(t2[1][2 * h], make_float2(v.z, v.w), q0);
+        mac(t2[1][2 * h + 1], make_float2(v.z, v.w), q1);
+      }
+    }
+    __syncthreads();
+  }
+#pragma unroll
+  for (int r = 0; r < 2; ++r)
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+      if (r0 + r < nm && col(i) < nm) T22out[(size_t)f * n2 + (r0 + r) * nm + col(i)] = t2[r][i];
+}
+
+// Refinement of one (frequency, right-hand side) per CTA: blockIdx.y = 0 the
+// axion beam's boost, 1 the reflection.  8 lanes a matrix row, 4 rows a warp,
+// P's rows then inverse(P)'s; a region's entries are loaded while the region
+// before is finished.  failed[f] is set when the iteration does not converge.
+constexpr int kRefineThreads = 512, kRefineMax = 8;
+__global__ void __launch_bounds__(kRefineThreads, 2)
+    k_refine(const float2* P, const float2* Pinv, const float2* X, const ChainRegionDF* cr, int nd, int nm,
+             const double2* emit, const double2* reflect, double2* boost, double2* refl, double* beta2, int* failed) {
+  constexpr int NW = kRefineThreads / 32, TASKS = 2 * 64 / 4 / NW;   // rows of 64 modes: 2 tasks of 4 a warp
+  __shared__ DFc vt[64], vb[64], pq[128], x[64], em[64];
+  __shared__ float red[2][2];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, l8 = lane & 7, f = blockIdx.x;
+  const bool back = blockIdx.y == 1;
+  const int n2 = nm * nm;
+  const DFc zero = {0.f, 0.f, 0.f, 0.f};
+  if (tid < nm) {
+    x[tid] = zero;
+    em[tid] = back ? zero : dfc_from(emit[tid]);
+  }
+  const float2* row[TASKS];
+  int out[TASKS];
+#pragma unroll
+  for (int t = 0; t < TASKS; ++t) {
+    const int r = 4 * (warp + NW * t) + (lane >> 3);
+    out[t] = r < 2 * nm ? r : -1;
+    row[t] = (r < nm ? P : Pinv) + (size_t)f * nd * n2 + (size_t)(r < nm ? r : r - nm) * nm;
+  }
+  float2 m[TASKS][8];
+  auto fetch = [&](int j) {
+#pragma unroll
+    for (int t = 0; t < TASKS; ++t)
+#pragma unroll
+      for (int i = 0; i < 8; ++i)
+        m[t][i] = out[t] >= 0 && l8 + 8 * i < nm ? row[t][(size_t)j * n2 + l8 + 8 * i] : make_float2(0.f, 0.f);
+  };
+  float last = 0.f;
+  bool ok = false;
+  for (int it = 0; it < kRefineMax && !ok; ++it) {
+    // the residual: the vector (reflect or 0, x) through the regions, nd - 1 to 1
+    fetch(nd - 1);
+    if (tid < nm) {
+      vt[tid] = back ? dfc_from(reflect[tid]) : zero;
+      vb[tid] = x[tid];
+    }
+    __syncthreads();
+    for (int j = nd - 1; j >= 1; --j) {
+#pragma unroll
+      for (int t = 0; t < TASKS; ++t) {
+        if (4 * (warp + NW * t) >= 2 * nm) continue;   // the whole warp
+        const DFc* v = out[t] < nm ? vt : vb;
+        float rh = 0.f, rl = 0.f, ih = 0.f, il = 0.f;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          const int k = l8 + 8 * i;
+          if (k >= nm) continue;
+          const DFc y = v[k];
+          const float2 a = m[t][i];
+          df_acc_prod(rh, rl, y.rh, a.x);
+          df_acc_prod(rh, rl, -y.ih, a.y);
+          df_acc_prod(ih, il, y.rh, a.y);
+          df_acc_prod(ih, il, y.ih, a.x);
+          rl = fmaf(y.rl, a.x, fmaf(-y.il, a.y, rl));
+          il = fmaf(y.rl, a.y, fmaf(y.il, a.x, il));
+        }
+        df_fast_two_sum(rh, rl);
+        df_fast_two_sum(ih, il);
+        DFc acc = {rh, rl, ih, il};
+#pragma unroll
+        for (int o = 1; o < 8; o <<= 1) acc = dfc_add(acc, dfc_shfl_xor(acc, o, 8));
+        if (l8 == 0 && out[t] >= 0) pq[out[t]] = acc;
+      }
+      if (j > 1) fetch(j - 1);
+      __syncthreads();
+      // G_j and the axion term: threads [0, 64) the top half, [64, 128) the bottom
+      if (tid < 128 && (tid & 63) < nm) {
+        const int k = tid & 63;
+        const ChainRegionDF& g = cr[j];
+        const DFc a = tid < 64 ? g.a : g.b, b = tid < 64 ? g.b : g.a;
+        DFc y = dfc_mul(g.inv2n, dfc_add(dfc_mul(a, pq[k]), dfc_mul(b, pq[nm + k])));
+        if (!back) y = dfc_add(y, dfc_mul(g.Sd, em[k]));
+        (tid < 64 ? vt : vb)[k] = y;
+      }
+      __syncthreads();
+    }
+    // d = X r, x -= d
+    if (tid < 4) red[tid >> 1][tid & 1] = 0.f;
+    __syncthreads();
+    for (int r = 4 * warp + (lane >> 3); r < (nm + 3) / 4 * 4; r += 4 * NW) {
+      float2 d = make_float2(0.f, 0.f);
+      if (r < nm)
+        for (int k = l8; k < nm; k += 8) {
+          const float2 a = X[(size_t)f * n2 + r * nm + k];
+          d.x = fmaf(a.x, vb[k].rh, fmaf(-a.y, vb[k].ih, d.x));
+          d.y = fmaf(a.x, vb[k].ih, fmaf(a.y, vb[k].rh, d.y));
+        }
+#pragma unroll
+      for (int o = 1; o < 8; o <<= 1) {
+        d.x += __shfl_xor_sync(0xffffffffu, d.x, o);
+        d.y += __shfl_xor_sync(0xffffffffu, d.y, o);
+      }
+      if (l8 == 0 && r < nm) {
+        const DFc n = dfc_add(x[r], DFc{-d.x, 0.f, -d.y, 0.f});
+        x[r] = n;
+        // non-negative floats order like their bits; a NaN orders above all
+        atomicMax(reinterpret_cast<int*>(&red[0][0]), __float_as_int(fabsf(d.x) + fabsf(d.y)));
+        atomicMax(reinterpret_cast<int*>(&red[0][1]), __float_as_int(fabsf(n.rh) + fabsf(n.ih)));
+      }
+    }
+    __syncthreads();
+    const float dn = red[0][0], xn = red[0][1];
+    // the next correction is about dn (dn / last); the first one (x itself) has no rate
+    if (dn == 0.f || (it > 0 && dn < 0.1f * last && dn * (dn / last) <= 1e-9f * xn)) ok = true;
+    else if (!(dn < INFINITY) || (it > 0 && !(dn < 0.5f * last))) break;   // not contracting
+    last = dn;
+    __syncthreads();
+  }
+  if (!ok) {
+    if (tid == 0) failed[f] = 1;
+    return;
+  }
+  if (tid < nm) (back ? refl : boost)[(size_t)f * nm + tid] = dfc_to_d(x[tid]);
+  if (tid == 0 && !back) {
+    double sum = 0.0;
+    for (int k = 0; k < nm; ++k) {
+      const double2 v = dfc_to_d(x[k]);
+      sum += v.x * v.x + v.y * v.y;
+    }
+    beta2[f] = sum;
+  }
+}
+
 // ---- transformer_trace_back: per-region amplitudes, one CTA per frequency ----
 // sol <- G_j blockdiag(P_j, inverse(P_j)) sol (+ S_j [emit; emit]), j = nd-1 .. 1,
 // starting from vcat(input, reflected) in the last region; every region's
@@ -1531,7 +1782,8 @@ __global__ void __launch_bounds__(256) k_trace_back(const PT* P, const PT* Pinv,
 template <typename C>
 __global__ void __launch_bounds__(256) k_final_solve(const C* T21g, const C* T22g, const double2* axg,
                                                      const double2* reflect, int nm, double2* boost,
-                                                     double2* refl, double* beta2, int* sing) {
+                                                     double2* refl, double* beta2, int* sing, const int* only) {
+  if (only && !only[blockIdx.x]) return;   // solved by refinement
   extern __shared__ __align__(16) unsigned char sm[];
   const int f = blockIdx.x, tid = threadIdx.x, nt = blockDim.x;
   const int w = nm + 2;
@@ -1653,11 +1905,12 @@ template <int NM>
 __global__ void __launch_bounds__(32) k_final_solve_warp(const double2* T21g, const double2* T22g,
                                                          const double2* axg, const double2* reflect, int nm,
                                                          double2* boost, double2* refl, double* beta2, int* sing,
-                                                         int nf) {
+                                                         int nf, const int* only) {
   constexpr unsigned FULL = 0xffffffffu;
   constexpr int SEG = 32 / NM;
   const int lane = threadIdx.x & 31, sl = lane % NM;
   const int first = blockIdx.x * SEG;
+  if (NM == 32 && only && !only[first]) return;   // solved by refinement (one frequency a warp)
   const int fi = first + lane / NM;
   const bool valid = fi < nf;
   const int f = valid ? fi : first;
@@ -2843,6 +3096,39 @@ static int tf_run_t(bf_handle* h, bf_stack* s, bf_modes* md, int nf, const doubl
   TCKS(T21.alloc(h, sizeof(double2) * (size_t)nf * nm * nm));
   TCKS(T22.alloc(h, sizeof(double2) * (size_t)nf * nm * nm));
   TCKS(ax.alloc(h, sizeof(double2) * (size_t)nf * nm));
+  // the chain's factors as double-floats
+  DBuf d_crd, d_failed, T21df, T22df;
+  int* failed = nullptr;   // refinement: the frequencies it leaves to the chain in double-float
+  auto split_regions = [&](DBuf& d) -> int {
+    static_assert(sizeof(ChainRegionDF) % sizeof(float4) == 0, "copied by 16 bytes");
+    std::vector<ChainRegionDF> v(nd);
+    auto split = [](double2 z) {
+      DFc r;
+      r.rh = (float)z.x;
+      r.rl = (float)(z.x - (double)r.rh);
+      r.ih = (float)z.y;
+      r.il = (float)(z.y - (double)r.ih);
+      return r;
+    };
+    for (int j = 1; j < nd; ++j) {
+      v[j].a = split(cr[j].a);
+      v[j].b = split(cr[j].b);
+      v[j].inv2n = split(cr[j].inv2n);
+      v[j].Sd = split(cr[j].S);
+      v[j].S = cr[j].S;
+      v[j].real = cr[j].a.y == 0.0 && cr[j].b.y == 0.0 && cr[j].inv2n.y == 0.0;
+    }
+    TCKS(d.alloc(h, sizeof(ChainRegionDF) * nd));
+    TCK(cudaMemcpyAsync(d.p, v.data(), sizeof(ChainRegionDF) * nd, cudaMemcpyHostToDevice, st));
+    return BF_OK;
+  };
+  if (reflect) {
+    TCKS(d_refl.alloc(h, sizeof(cd) * nm));
+    TCK(cudaMemcpyAsync(d_refl.p, reflect, sizeof(cd) * nm, cudaMemcpyHostToDevice, st));
+  }
+  TCKS(boost.alloc(h, sizeof(cd) * (size_t)nf * nm));
+  if (reflect) TCKS(refl.alloc(h, sizeof(cd) * (size_t)nf * nm));
+  TCKS(b2.alloc(h, sizeof(double) * nf));
   if constexpr (fp64) {
     // rows per CTA: as many CTAs as SMs when the frequencies alone leave SMs
     // idle, about 256 entries a CTA otherwise
@@ -2862,26 +3148,7 @@ static int tf_run_t(bf_handle* h, bf_stack* s, bf_modes* md, int nf, const doubl
         ax.as<double2>());
     TCK(cudaGetLastError());
   } else if (nm <= 16 && nd <= 512) {
-    std::vector<ChainRegionDF> crd(nd);
-    static_assert(sizeof(ChainRegionDF) % sizeof(float4) == 0, "copied by 16 bytes");
-    auto split = [](double2 v) {
-      DFc r;
-      r.rh = (float)v.x;
-      r.rl = (float)(v.x - (double)r.rh);
-      r.ih = (float)v.y;
-      r.il = (float)(v.y - (double)r.ih);
-      return r;
-    };
-    for (int j = 1; j < nd; ++j) {
-      crd[j].a = split(cr[j].a);
-      crd[j].b = split(cr[j].b);
-      crd[j].inv2n = split(cr[j].inv2n);
-      crd[j].S = cr[j].S;
-      crd[j].real = cr[j].a.y == 0.0 && cr[j].b.y == 0.0 && cr[j].inv2n.y == 0.0;
-    }
-    DBuf d_crd;
-    TCKS(d_crd.alloc(h, sizeof(ChainRegionDF) * nd));
-    TCK(cudaMemcpyAsync(d_crd.p, crd.data(), sizeof(ChainRegionDF) * nd, cudaMemcpyHostToDevice, st));
+    TCKS(split_regions(d_crd));
     auto run = [&](auto NMc) -> int {
       constexpr int NM = decltype(NMc)::value, RW = 32 / NM;
       const int tasks = nf * ((nm + RW - 1) / RW);
@@ -2896,19 +3163,51 @@ static int tf_run_t(bf_handle* h, bf_stack* s, bf_modes* md, int nf, const doubl
     };
     TCKS(nm <= 8 ? run(std::integral_constant<int, 8>()) : run(std::integral_constant<int, 16>()));
   } else {
-    DBuf T21df, T22df, Wdf;
+    DBuf Wdf;
     size_t smem = (sizeof(DFc) * 2 + sizeof(float2) * 2) * nm * nm + (sizeof(double2) + sizeof(DFc)) * nm;
     const bool t_in_smem = smem + sizeof(DFc) * 2 * nm * nm <= 160 * 1024;
     const bool par_axion = t_in_smem && smem + sizeof(DFc) * 3 * nm * nm <= 160 * 1024;
     if (t_in_smem) {
       smem += sizeof(DFc) * (par_axion ? 3 : 2) * nm * nm;
     } else {
-      TCKS(T21df.alloc(h, sizeof(DFc) * (size_t)nf * nm * nm));
-      TCKS(T22df.alloc(h, sizeof(DFc) * (size_t)nf * nm * nm));
+      TCKS(T21df.ensure(h, sizeof(DFc) * (size_t)nf * nm * nm));
+      TCKS(T22df.ensure(h, sizeof(DFc) * (size_t)nf * nm * nm));
       // the axion terms go to global scratch, so that their row sums (in k
       // order) are a short chain beside the products instead of a long one
       // before them
       TCKS(Wdf.alloc(h, sizeof(DFc) * (size_t)nf * nm * nm));
+    }
+    if (nm > 16 && nm <= 64) {
+      // T22 in complex64 and its inverse share the buffers of the double-float
+      // chain, which runs after them, if at all
+      const size_t n22 = sizeof(float2) * (size_t)nf * nm * nm;
+      TCKS(T21df.ensure(h, n22));
+      TCKS(T22df.ensure(h, n22));
+      TCKS(d_failed.alloc(h, sizeof(int) * (nf + 1)));   // and a singularity word nobody reads
+      TCK(cudaMemsetAsync(d_failed.p, 0, sizeof(int) * (nf + 1), st));
+      failed = d_failed.as<int>();
+      TCKS(split_regions(d_crd));
+      auto run = [&](auto NBc) -> int {
+        constexpr int NB = decltype(NBc)::value;
+        const size_t sm32 = sizeof(float2) * (4 * NB * NB + 2 * NB * (NB + 2));
+        TCK(cudaFuncSetAttribute(k_chain_f32<NB>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxDynSmem));
+        bf::note_launch();
+        k_chain_f32<NB><<<nf, (NB / 2) * (NB / 4), sm32, st>>>(Pd, Pinv.as<D2>(), d_crd.as<ChainRegionDF>(), nd, nm,
+                                                              T21df.as<float2>());
+        TCK(cudaGetLastError());
+        bf::note_launch();
+        k_invert_reg<NB><<<dim3(1, nf), (NB / 4) * (NB / 4), 0, st>>>(T21df.as<float2>(), T22df.as<float2>(), 1, 0, nm,
+                                                                     failed + nf);
+        TCK(cudaGetLastError());
+        return BF_OK;
+      };
+      TCKS(nm <= 32 ? run(std::integral_constant<int, 32>()) : run(std::integral_constant<int, 64>()));
+      bf::note_launch();
+      k_refine<<<dim3(nf, reflect ? 2 : 1), kRefineThreads, 0, st>>>(
+          Pd, Pinv.as<D2>(), T22df.as<float2>(), d_crd.as<ChainRegionDF>(), nd, nm, d_em.as<double2>(),
+          reflect ? d_refl.as<double2>() : nullptr, boost.as<double2>(), reflect ? refl.as<double2>() : nullptr,
+          b2.as<double>(), failed);
+      TCK(cudaGetLastError());
     }
     TCK(cudaFuncSetAttribute(k_chain_df, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxDynSmem));
     bf::note_launch();
@@ -2919,23 +3218,16 @@ static int tf_run_t(bf_handle* h, bf_stack* s, bf_modes* md, int nf, const doubl
     k_chain_df<<<nf, nthr, smem, st>>>(Pd, Pinv.as<D2>(), d_cr.as<ChainRegion>(), nd, nm, d_em.as<double2>(),
                                       t_in_smem ? nullptr : T21df.as<DFc>(), t_in_smem ? nullptr : T22df.as<DFc>(),
                                       ax.as<double2>(), T21.as<double2>(),
-                                      T22.as<double2>(), par_axion ? 1 : 0, t_in_smem ? nullptr : Wdf.as<DFc>());
+                                      T22.as<double2>(), par_axion ? 1 : 0, t_in_smem ? nullptr : Wdf.as<DFc>(), failed);
     TCK(cudaGetLastError());
   }
-  if (reflect) {
-    TCKS(d_refl.alloc(h, sizeof(cd) * nm));
-    TCK(cudaMemcpyAsync(d_refl.p, reflect, sizeof(cd) * nm, cudaMemcpyHostToDevice, st));
-  }
-  TCKS(boost.alloc(h, sizeof(cd) * (size_t)nf * nm));
-  if (reflect) TCKS(refl.alloc(h, sizeof(cd) * (size_t)nf * nm));
-  TCKS(b2.alloc(h, sizeof(double) * nf));
   if (nm <= 32) {
     auto run = [&](auto NMc) -> int {
       constexpr int NM = decltype(NMc)::value, SEG = 32 / NM;
       bf::note_launch();
       k_final_solve_warp<NM><<<(nf + SEG - 1) / SEG, 32, 0, st>>>(
           T21.as<double2>(), T22.as<double2>(), ax.as<double2>(), reflect ? d_refl.as<double2>() : nullptr, nm,
-          boost.as<double2>(), reflect ? refl.as<double2>() : nullptr, b2.as<double>(), d_sing + 1, nf);
+          boost.as<double2>(), reflect ? refl.as<double2>() : nullptr, b2.as<double>(), d_sing + 1, nf, failed);
       TCK(cudaGetLastError());
       return BF_OK;
     };
@@ -2948,7 +3240,8 @@ static int tf_run_t(bf_handle* h, bf_stack* s, bf_modes* md, int nf, const doubl
     bf::note_launch();
     k_final_solve<double2><<<nf, 256, smem, st>>>(T21.as<double2>(), T22.as<double2>(), ax.as<double2>(),
                                              reflect ? d_refl.as<double2>() : nullptr, nm, boost.as<double2>(),
-                                             reflect ? refl.as<double2>() : nullptr, b2.as<double>(), d_sing + 1);
+                                             reflect ? refl.as<double2>() : nullptr, b2.as<double>(), d_sing + 1,
+                                             failed);
     TCK(cudaGetLastError());
   }
   DBuf d_ant, d_cpl;

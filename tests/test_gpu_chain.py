@@ -50,3 +50,33 @@ def test_mode_counts_vs_oracle(B, nm, nf, eps):
         for i, k in enumerate(check):
             assert rel(boost[k], ref[i][0]) < tol and rel(back[k], ref[i][1]) < tol, (precision, k)
             assert rel(alone[k], ref[i][0]) < tol, (precision, k)
+
+
+@pytest.mark.parametrize("nm,ndisk,eps", [(17, 6, 24.0), (32, 6, 24.0), (33, 6, 9.4 + 0.01j), (64, 6, 24.0),
+                                          (17, 10, 60.0), (40, 10, 60.0), (64, 10, 60.0)])
+def test_refined_boundary_solve(B, nm, ndisk, eps):
+    """The mixed boundary solve by refinement (17 to 64 modes) on injected
+    matrices that complex64 holds, and inverts, exactly (permutations times
+    powers of i), so that its result is as exact as the double-float residual:
+    6 disks refine (cond(T22) ~ 3e3), 10 disks of eps 60 have a cond(T22) of ~1e7,
+    beyond complex64, and fall back to the double-float chain.  Double-float
+    carries ~48 bits: 1e-14 times cond(T22), 1e-7 here."""
+    n = 24
+    rng = np.random.default_rng([nm, ndisk])
+    X = W.symmetric_grid(n)
+    distance, e, _, _ = W.booster(ndisk, np.full(ndisk, 8e-3), eps_disk=eps)
+    nd = len(e)
+    pm = np.zeros((nd, nm, nm), dtype=complex)
+    for j in range(nd):
+        pm[j, np.arange(nm), rng.permutation(nm)] = 1j ** rng.integers(0, 4, nm)
+    pats, kt = W.lg_modes(X, X, nm, 0.05, 0.3)
+    c, co = B.SeedCoordinateSystem(X=X, Y=X), O.seed_coordinate_system(X=X, Y=X)
+    kw = dict(ThreeDim=True, Mmax=nm, Lmax=0, diskR=0.3, pattern_input=pats, kT_arr=kt)
+    m, mo = B.SeedModes(c, **kw), O.seed_modes(co, **kw)
+    geo = dict(diskno=ndisk, distance=distance, epsilon=e)
+    emit, refl = rng.standard_normal((2, nm)) + 1j * rng.standard_normal((2, nm))
+    args = dict(f=20e9, diskR=0.3, emit=emit, reflect=refl, propagation_matrices=pm)
+    ref = O.transformer(O.seed_setup_boundaries(co, **geo), co, mo, **args)
+    got = B.transformer(B.SeedSetupBoundaries(c, **geo), c, m, precision="mixed", **args)
+    for x, y in zip(got, ref):
+        assert rel(x, y) < 1e-6
