@@ -614,6 +614,70 @@ __global__ void k_build_diag(double2* DG, const double2* K0, int nf, int npx, co
   DG[i] = dexp_c(kz.y * g.dz, -kz.x * g.dz);
 }
 
+// gram[m][m'] = sum_s conj(Psi_m(x_s)) Psi_m'(x_s) over the support pixels in FP64 (Hermitian), one CTA of 256
+// threads a pair m <= m', summed in k_rowsum's order
+__global__ void k_gram(double2* gram, const double2* pat, const int* supp, int Kd, int nm, int npix) {
+  __shared__ double2 red[256];
+  int m = 0, t = blockIdx.x;
+  while (t >= nm - m) t -= nm - m++;
+  const int mp = m + t;
+  double2 acc = make_double2(0.0, 0.0);
+  for (int s = threadIdx.x; s < Kd; s += blockDim.x) {
+    const double2 a = pat[(size_t)m * npix + supp[s]], b = pat[(size_t)mp * npix + supp[s]];
+    acc.x += a.x * b.x + a.y * b.y;
+    acc.y += a.x * b.y - a.y * b.x;
+  }
+  red[threadIdx.x] = acc;
+  __syncthreads();
+  for (int w = blockDim.x / 2; w > 0; w >>= 1) {
+    if (threadIdx.x < w) red[threadIdx.x] = bf::cadd(red[threadIdx.x], red[threadIdx.x + w]);
+    __syncthreads();
+  }
+  if (threadIdx.x == 0) {
+    gram[(size_t)mp * nm + m] = make_double2(red[0].x, -red[0].y);
+    gram[(size_t)m * nm + mp] = red[0];
+  }
+}
+
+// the same from the sums g[2t step], g[(2t + 1) step] of the real rows of the mixed paths' V, whose rounding it then
+// shares
+__global__ void k_gram_from_rows(double2* gram, const double* g, int step, const int2* tri, int T, int nm) {
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= T) return;
+  const int2 mp = tri[t];
+  gram[(size_t)mp.y * nm + mp.x] = make_double2(g[2 * t * step], -g[(2 * t + 1) * step]);
+  gram[(size_t)mp.x * nm + mp.y] = make_double2(g[2 * t * step], g[(2 * t + 1) * step]);
+}
+
+// P of the disks without tilt and surface map.  Their pixel factor is 1 at every
+// pixel and frequency, so the overlap is the modes' Gram matrix and
+// P = diag(exp(-i kz_m dz)) gram: no operand and no GEMM, and the diagonal once
+// for all disks of one permittivity and thickness (toff: the types' ranges in
+// `members`).  A CTA takes a (frequency, type) and a slice of the entries; bound
+// by the writes.  20 disks: 8 modes, 256
+// frequencies 8 us for 152 (operand, GEMM, scatter); FP64, 28 modes, 29 frequencies 10 us for 1380.
+template <typename PT>
+__global__ void __launch_bounds__(256) k_flat_disks(PT* P, const double2* gram, const double* freqs, int nf, int nrep,
+                                                    int nd, int nm, const double2* kt, const RegionT* regs,
+                                                    const int* members, const int* toff) {
+  extern __shared__ double2 diag[];
+  const int f = blockIdx.x, t0 = toff[blockIdx.y], t1 = toff[blockIdx.y + 1], n2 = nm * nm;
+  const RegionT g = regs[members[t0]];
+  for (int m = threadIdx.x; m < nm; m += blockDim.x) {
+    const double2 k0 = k0_c(kC / freqs[f], g.er, g.ei), t = kt[m];
+    const double2 k0sq = make_double2(k0.x * k0.x - k0.y * k0.y, k0.x * k0.y + k0.y * k0.x);
+    const double2 ktsq = make_double2(t.x * t.x - t.y * t.y, t.x * t.y + t.y * t.x);
+    const double2 kz = dsqrt_c(k0sq.x - ktsq.x, k0sq.y - ktsq.y);
+    diag[m] = dexp_c(kz.y * g.dz, -kz.x * g.dz);
+  }
+  __syncthreads();
+  for (int e = blockIdx.z * blockDim.x + threadIdx.x; e < n2; e += gridDim.z * blockDim.x) {
+    const PT v = dto<PT>(bf::cmul(diag[e / nm], gram[e]));
+    for (int r = 0; r < nrep; ++r)
+      for (int i = t0; i < t1; ++i) P[((size_t)(r * nf + f) * nd + members[i]) * n2 + e] = v;
+  }
+}
+
 // P[f][j][m][m'] from a class GEMM output G[mm'][f*ncols + col]; pixel-class
 // disk regions get the propagation diag(exp(-i kz_m dz)) from the left.
 template <typename PT>
@@ -935,18 +999,20 @@ __global__ void __launch_bounds__((NB / 4) * (NB / 4)) k_invert_reg(const float2
   for (int e = tid; e < nm * nm; e += NT) Pinv[off + e] = outs[e];
 }
 
-// Group solves: the inverses of regions jl[0 .. njl) of request 0 (frequencies
-// [0, nf)) copied to requests 1 .. nreq-1, whose matrices there are the same.
+// Inverses copied instead of computed again: region to.x of every request gets
+// that of region to.y of request 0 (frequencies [0, nf)), whose matrix is the
+// same: the disks of a group's requests, and disks of one permittivity and
+// thickness without tilt and surface map.
 template <typename C>
-__global__ void k_copy_inverses(C* Pinv, int nd, int nm, int nf, int nreq, const int* jl, int njl) {
+__global__ void k_copy_inverses(C* Pinv, int nd, int nm, int nf, int nreq, const int2* tos, int nto) {
   const size_t n2 = (size_t)nm * nm;
-  const size_t per = (size_t)nf * njl * n2;   // entries of request 0 to copy
-  const size_t total = per * (nreq - 1);
+  const size_t total = (size_t)nf * nto * n2;
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
-    const size_t r = 1 + i / per, q = i % per;
-    const size_t e = q % n2, fj = q / n2;
-    const int f = (int)(fj / njl), j = jl[fj % njl];
-    Pinv[(((r * nf + f) * nd) + j) * n2 + e] = Pinv[(((size_t)f * nd) + j) * n2 + e];
+    const size_t e = i % n2, fj = i / n2;
+    const int f = (int)(fj / nto);
+    const int2 to = tos[fj % nto];
+    const C v = Pinv[((size_t)f * nd + to.y) * n2 + e];
+    for (int r = to.x == to.y ? 1 : 0; r < nreq; ++r) Pinv[((size_t)(r * nf + f) * nd + to.x) * n2 + e] = v;
   }
 }
 
@@ -2044,6 +2110,7 @@ struct TfCache {
   // [Mp][Kdp] (rows padded to a multiple of 128, K to a multiple of 32) and
   // their FP64 row sums (gW, gV)
   DBuf Wh, Wl, Vh, Vl, gW, gV;
+  DBuf gram;  // the modes' Gram matrix over the support pixels [nm][nm] (FP64)
   DBuf KT2;   // kx^2 + ky^2 at each orbit representative (FP32)
   int Kp = 0, Kdp = 0, Mp = 0;
   std::vector<int2> rep_h;
@@ -2054,10 +2121,13 @@ static size_t tf_cache_bytes(const void* p) {
   const TfCache* c = static_cast<const TfCache*>(p);
   size_t b = 0;
   for (const DBuf* d : {&c->W, &c->V, &c->Vr, &c->Wr, &c->tri, &c->rep, &c->supp, &c->U, &c->Phi, &c->members,
-                        &c->Wh, &c->Wl, &c->Vh, &c->Vl, &c->gW, &c->gV, &c->KT2})
+                        &c->Wh, &c->Wl, &c->Vh, &c->Vl, &c->gW, &c->gV, &c->gram, &c->KT2})
     b += d->p ? d->n : 0;
   return b;
 }
+
+static thread_local double g_tf_gemm_flops = 0.0;   // executed real flops of the class GEMMs of this thread's last solve
+static int launch_rgemm(bf_handle* h, const float* A, const float2* B, double2* Hm, int R, int K, int N);
 
 static int tf_setup(bf_handle* h, bf_stack* s, bf_modes* md, int mode, TfCache** out) {
   const bool fp64 = mode == 0;
@@ -2072,7 +2142,9 @@ static int tf_setup(bf_handle* h, bf_stack* s, bf_modes* md, int mode, TfCache**
   // which a stack changes after creation (bf_stack_set_distance moves the
   // disks), so gap updates of an optimiser reuse them.
   if (c.modes_id == md->id && c.mode == mode) return BF_OK;
-  for (DBuf* d : {&c.W, &c.V, &c.Vr, &c.Wr, &c.tri, &c.Wh, &c.Wl, &c.Vh, &c.Vl, &c.gW, &c.gV, &c.KT2}) d->release();
+  for (DBuf* d : {&c.W, &c.V, &c.Vr, &c.Wr, &c.tri, &c.Wh, &c.Wl, &c.Vh, &c.Vl, &c.gW, &c.gV, &c.gram,
+                  &c.KT2})
+    d->release();
   cudaStream_t st = h->stream();
   const int nx = s->nx, ny = s->ny, nm = md->nm;
   const size_t npix = (size_t)nx * ny;
@@ -2213,6 +2285,7 @@ static int tf_setup(bf_handle* h, bf_stack* s, bf_modes* md, int mode, TfCache**
   TCKS(c.supp.alloc(h, sizeof(int) * supp.size()));
   TCK(cudaMemcpyAsync(c.supp.p, supp.data(), sizeof(int) * supp.size(), cudaMemcpyHostToDevice, st));
   c.Kdp = (c.Kd + 31) / 32 * 32;
+  TCKS(c.gram.alloc(h, sizeof(double2) * nm * nm));
   {
     dim3 grid(blocks_for(c.Kd), nm * nm);
     bf::note_launch();
@@ -2220,10 +2293,22 @@ static int tf_setup(bf_handle* h, bf_stack* s, bf_modes* md, int mode, TfCache**
       TCKS(c.V.alloc(h, csz * (size_t)nm * nm * c.Kd));
       k_build_v<double2><<<grid, 256, 0, st>>>(c.V.as<double2>(), md->d_pat, c.supp.as<int>(), c.Kd, nm,
                                                (int)npix);
+      TCK(cudaGetLastError());
+      bf::note_launch();
+      k_gram<<<nm * (nm + 1) / 2, 256, 0, st>>>(c.gram.as<double2>(), md->d_pat, c.supp.as<int>(), c.Kd, nm,
+                                                (int)npix);
     } else if (mode == 1) {
       TCKS(c.Vr.alloc(h, sizeof(float) * 2 * (size_t)c.T * c.Kd));
       k_build_vr<<<dim3(blocks_for(c.Kd), c.T), 256, 0, st>>>(c.Vr.as<float>(), md->d_pat, c.supp.as<int>(),
                                                                c.tri.as<int2>(), c.Kd, (int)npix);
+      TCK(cudaGetLastError());
+      // the rows' sums in the GEMM's own rounding: its column of a factor 1
+      const std::vector<float2> ones(c.Kd, make_float2(1.f, 0.f));
+      DBuf one;
+      TCKS(one.alloc(h, sizeof(float2) * c.Kd));
+      TCK(cudaMemcpyAsync(one.p, ones.data(), sizeof(float2) * c.Kd, cudaMemcpyHostToDevice, st));
+      TCKS(c.gV.alloc(h, sizeof(double2) * 2 * c.T));
+      TCKS(launch_rgemm(h, c.Vr.as<float>(), one.as<float2>(), c.gV.as<double2>(), 2 * c.T, c.Kd, 1));
     } else {
       const size_t n = (size_t)c.Mp * c.Kdp;
       TCKS(c.Vh.alloc(h, sizeof(float) * n));
@@ -2242,6 +2327,12 @@ static int tf_setup(bf_handle* h, bf_stack* s, bf_modes* md, int mode, TfCache**
       k_rowsum<<<2 * c.T, 256, 0, st>>>(c.gV.as<double>(), Vd.as<double>(), c.Kd);
     }
     TCK(cudaGetLastError());
+    if (!fp64) {
+      bf::note_launch();
+      k_gram_from_rows<<<blocks_for(c.T), 256, 0, st>>>(c.gram.as<double2>(), c.gV.as<double>(), mode == 1 ? 2 : 1,
+                                                        c.tri.as<int2>(), c.T, nm);
+      TCK(cudaGetLastError());
+    }
   }
   TCK(cudaStreamSynchronize(st));
   c.U.release();
@@ -2252,7 +2343,6 @@ static int tf_setup(bf_handle* h, bf_stack* s, bf_modes* md, int mode, TfCache**
   return BF_OK;
 }
 
-static thread_local double g_tf_gemm_flops = 0.0;   // executed real flops of the class GEMMs of this thread's last solve
 // CUDA events around each class-GEMM kernel of this thread's solve (profiling only)
 static thread_local std::vector<std::pair<cudaEvent_t, cudaEvent_t>> g_gemm_ev;
 static void gemm_ev_begin(bf_handle* h) {
@@ -2442,6 +2532,12 @@ static int tc_class_gemm(bf_handle* h, const float* Ah, const float* Al, int Mp,
   return BF_OK;
 }
 
+// A disk whose tilt and surface factor is 1 everywhere
+static bool flat_disk(const bf_stack* s, const RegionT& r, int j) {
+  return r.klass == 1 && r.tx == 0.0 && r.ty == 0.0 && !(s->d_surf && s->surf_nonzero[j]);
+}
+static bool same_disk(const RegionT& a, const RegionT& b) { return a.er == b.er && a.ei == b.ei && a.dz == b.dz; }
+
 // Propagation matrices of regions [j0, nd) for all frequencies into
 // P[f][j][m][m'] stored as S, which is also the operand storage of the class
 // GEMMs: double2 (FP64 path) or float2 (mixed path).  A group solve (nreq > 1)
@@ -2459,10 +2555,11 @@ static int tf_propagation_matrices(bf_handle* h, bf_stack* s, bf_modes* md, TfCa
   cudaStream_t st = h->stream();
   const int nd = s->nd, nm = md->nm, nx = s->nx, ny = s->ny;
   const size_t npix = (size_t)nx * ny;
-  std::vector<int> kreg, preg, freg;
+  std::vector<int> kreg, preg, freg, flat;
   for (int j = j0; j < nd; ++j) {
     if (regs[j].klass == 0) kreg.push_back(j);
     else if (regs[j].klass == 3) freg.push_back(j);
+    else if (flat_disk(s, regs[j], j)) flat.push_back(j);
     else preg.push_back(j);
   }
   int* tc_err = reinterpret_cast<int*>(h->d_scalar + 2);   // set by the tensor-core GEMM on a wait timeout
@@ -2567,6 +2664,31 @@ static int tf_propagation_matrices(bf_handle* h, bf_stack* s, bf_modes* md, TfCa
       }
       TCK(cudaGetLastError());
     }
+  }
+  if (!flat.empty()) {
+    std::vector<int> lists, toff = {0};   // regions by type, then the types' offsets
+    for (size_t i = 0; i < flat.size(); ++i) {
+      if (flat[i] < 0) continue;
+      for (size_t k = flat.size(); k-- > i + 1;)
+        if (flat[k] >= 0 && same_disk(regs[flat[i]], regs[flat[k]])) {
+          lists.push_back(flat[k]);
+          flat[k] = -1;
+        }
+      lists.push_back(flat[i]);
+      toff.push_back((int)lists.size());
+    }
+    const int ntypes = (int)toff.size() - 1, nflat = (int)lists.size();
+    lists.insert(lists.end(), toff.begin(), toff.end());
+    DBuf d_lists;
+    TCKS(d_lists.alloc(h, sizeof(int) * lists.size()));
+    TCK(cudaMemcpyAsync(d_lists.p, lists.data(), sizeof(int) * lists.size(), cudaMemcpyHostToDevice, st));
+    // slices of the entries only where the frequencies leave SMs idle: each slice computes the diagonal again
+    const int slices = std::max(1, std::min((nm * nm + 255) / 256, 2 * 152 / std::max(1, nf * ntypes)));
+    bf::note_launch();
+    k_flat_disks<S><<<dim3(nf, ntypes, slices), 256, sizeof(double2) * nm, st>>>(
+        P.as<S>(), c.gram.as<double2>(), d_freq.as<double>(), nf, nreq, nd, nm, d_kt.as<double2>(), dr,
+        d_lists.as<int>(), d_lists.as<int>() + nflat);
+    TCK(cudaGetLastError());
   }
   // pixel class: one GEMM V * E
   if (!preg.empty()) {
@@ -3015,30 +3137,42 @@ static int tf_run_t(bf_handle* h, bf_stack* s, bf_modes* md, int nf, const doubl
     TCK(cudaGetLastError());
     return BF_OK;
   };
-  if (nreq > 1) {
-    // a group: request 0 inverts every region; the others only their own
-    // (k-space) air regions and take the disk regions' inverses from request 0
+  {
+    // request 0 inverts every region but the disks that equal an earlier one;
+    // the others of a group only their own (k-space) air regions
     const int nf0 = nf / nreq;
-    std::vector<int> own, shared;
-    for (int j = 1; j < nd; ++j) (regs[j].klass == 0 ? own : shared).push_back(j);
-    DBuf d_own, d_shared;
-    TCKS(invert(0, nf0, nullptr, 0));
-    if (!own.empty()) {
+    std::vector<int> first, own;
+    std::vector<int2> copies;
+    for (int j = 1; j < nd; ++j) {
+      int same = j;
+      if (!pm && !P_dev && flat_disk(s, regs[j], j))
+        for (same = 1; same < j && !(flat_disk(s, regs[same], same) && same_disk(regs[same], regs[j]));) ++same;
+      if (same == j) first.push_back(j);
+      if (same != j || (nreq > 1 && regs[j].klass != 0)) copies.push_back(make_int2(j, same));
+      if (regs[j].klass == 0) own.push_back(j);
+    }
+    DBuf d_first, d_own, d_copies;
+    if ((int)first.size() < nd - 1) {
+      TCKS(d_first.alloc(h, sizeof(int) * first.size()));
+      TCK(cudaMemcpyAsync(d_first.p, first.data(), sizeof(int) * first.size(), cudaMemcpyHostToDevice, st));
+      TCKS(invert(0, nf0, d_first.as<int>(), (int)first.size()));
+    } else {
+      TCKS(invert(0, nf0, nullptr, 0));
+    }
+    if (nreq > 1 && !own.empty()) {
       TCKS(d_own.alloc(h, sizeof(int) * own.size()));
       TCK(cudaMemcpyAsync(d_own.p, own.data(), sizeof(int) * own.size(), cudaMemcpyHostToDevice, st));
       TCKS(invert(nf0, nf - nf0, d_own.as<int>(), (int)own.size()));
     }
-    if (!shared.empty()) {
-      TCKS(d_shared.alloc(h, sizeof(int) * shared.size()));
-      TCK(cudaMemcpyAsync(d_shared.p, shared.data(), sizeof(int) * shared.size(), cudaMemcpyHostToDevice, st));
-      const size_t total = (size_t)nf0 * shared.size() * nm * nm * (nreq - 1);
+    if (!copies.empty()) {
+      TCKS(d_copies.alloc(h, sizeof(int2) * copies.size()));
+      TCK(cudaMemcpyAsync(d_copies.p, copies.data(), sizeof(int2) * copies.size(), cudaMemcpyHostToDevice, st));
+      const size_t total = (size_t)nf0 * copies.size() * nm * nm;
       bf::note_launch();
       k_copy_inverses<D2><<<(unsigned)std::min<size_t>(blocks_for(total), 1u << 20), 256, 0, st>>>(
-          Pinv.as<D2>(), nd, nm, nf0, nreq, d_shared.as<int>(), (int)shared.size());
+          Pinv.as<D2>(), nd, nm, nf0, nreq, d_copies.as<int2>(), (int)copies.size());
       TCK(cudaGetLastError());
     }
-  } else {
-    TCKS(invert(0, nf, nullptr, 0));
   }
   // chain coefficients: step j uses n_left = sqrt(eps[j]), n_right = sqrt(eps[j-1])
   std::vector<ChainRegion> cr(nd);
