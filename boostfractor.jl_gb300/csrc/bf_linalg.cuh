@@ -162,6 +162,68 @@ __global__ void __launch_bounds__(256, 1) k_cgemm_c64(const float2* __restrict__
     }
 }
 
+// Hm = A B with real FP64 A [R][K] and complex128 B [K][N].  Bound by the FP64
+// pipe (two lanes an SM and clock), so small tiles that share the work out evenly
+// count for more than reuse: 32 rows x 16 columns a CTA, 2 x 2 a thread.  118 x
+// 609 x 351: 181 us; the complex product of all 784 pairs took 2430 us.
+static __global__ void __launch_bounds__(128) k_rcgemm_d(const double* __restrict__ A, const double2* __restrict__ B,
+                                                  double2* __restrict__ Hm, int R, int K, int N) {
+  constexpr int TM = 32, TN = 16, TK = 16;
+  __shared__ double As[2][TK][TM + 1];
+  __shared__ double2 Bs[2][TK][TN];
+  const int tid = threadIdx.x, tr = tid / 8, tc = tid % 8;
+  const int r0 = blockIdx.y * TM, c0 = blockIdx.x * TN;
+  double pa[4];
+  double2 pb[2];
+  auto fetch = [&](int k0) {
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const int e = tid + 128 * q, r = r0 + e / TK, k = k0 + e % TK;
+      pa[q] = r < R && k < K ? A[(size_t)r * K + k] : 0.0;
+    }
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+      const int e = tid + 128 * q, k = k0 + e / TN, c = c0 + e % TN;
+      pb[q] = k < K && c < N ? B[(size_t)k * N + c] : make_double2(0.0, 0.0);
+    }
+  };
+  auto put = [&](int b) {
+#pragma unroll
+    for (int q = 0; q < 4; ++q) As[b][(tid + 128 * q) % TK][(tid + 128 * q) / TK] = pa[q];
+#pragma unroll
+    for (int q = 0; q < 2; ++q) Bs[b][(tid + 128 * q) / TN][(tid + 128 * q) % TN] = pb[q];
+  };
+  double2 acc[2][2] = {};
+  fetch(0);
+  put(0);
+  __syncthreads();
+  for (int k0 = 0, b = 0; k0 < K; k0 += TK, b ^= 1) {
+    const bool more = k0 + TK < K;
+    if (more) fetch(k0 + TK);
+#pragma unroll
+    for (int k = 0; k < TK; ++k) {
+      const double a[2] = {As[b][k][tr], As[b][k][tr + 16]};
+      const double2 v[2] = {Bs[b][k][tc], Bs[b][k][tc + 8]};
+#pragma unroll
+      for (int i = 0; i < 2; ++i)
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+          acc[i][j].x = fma(a[i], v[j].x, acc[i][j].x);
+          acc[i][j].y = fma(a[i], v[j].y, acc[i][j].y);
+        }
+    }
+    if (more) put(b ^ 1);
+    __syncthreads();
+  }
+#pragma unroll
+  for (int i = 0; i < 2; ++i)
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+      const int r = r0 + tr + 16 * i, c = c0 + tc + 8 * j;
+      if (r < R && c < N) Hm[(size_t)r * N + c] = acc[i][j];
+    }
+}
+
 // Real-by-complex GEMM Cout[r][c] = sum_k A[r][k] B[k][c]: A real (FP32),
 // B complex64, one FP32 product per term and accumulator, summed like
 // k_cgemm_c64 (FP32 over a 16-term K tile, TwoSum-folded into double-float).

@@ -21,6 +21,7 @@
 #include <algorithm>
 #include <array>
 #include <atomic>
+#include <cfloat>
 #include <cmath>
 #include <cstdio>
 #include <cstring>
@@ -170,10 +171,10 @@ __global__ void k_build_v(C* V, const double2* pat, const int* supp, int Kd, int
   V[(size_t)mm * Kd + s] = dto<C>(make_double2(a.x * b.x + a.y * b.y, a.x * b.y - a.y * b.x));
 }
 
-// Upper triangle of W as real rows (valid when W is Hermitian in the mode
-// pair: Phi = U, every mode zero outside the mask): pair t = (m, m') gives
-// Wr[2t][o] = Re W[mm'][o], Wr[2t+1][o] = Im W[mm'][o], summed like k_build_w.
-__global__ void k_build_wr(float* Wr, const double2* U, const double2* Phi, const int* members, const int2* tri,
+// Upper triangle of W as real rows in FP64 (valid when W is Hermitian in the
+// mode pair: Phi = U, every mode zero outside the mask): pair t = (m, m') gives
+// rows 2t and 2t + 1, Re and Im W[mm'][o], summed like k_build_w.
+__global__ void k_build_wr(double* Wr, const double2* U, const double2* Phi, const int* members, const int2* tri,
                            int K, int msz, int npix, double scale) {
   const int o = blockIdx.x * blockDim.x + threadIdx.x;
   const int t = blockIdx.y;
@@ -187,8 +188,15 @@ __global__ void k_build_wr(float* Wr, const double2* U, const double2* Phi, cons
     acc.x += u.x * p.x + u.y * p.y;
     acc.y += u.x * p.y - u.y * p.x;
   }
-  Wr[(size_t)(2 * t) * K + o] = (float)(acc.x * scale);
-  Wr[(size_t)(2 * t + 1) * K + o] = (float)(acc.y * scale);
+  Wr[(size_t)(2 * t) * K + o] = acc.x * scale;
+  Wr[(size_t)(2 * t + 1) * K + o] = acc.y * scale;
+}
+
+// out[r] = Ad[rows[r]] as T
+template <typename T>
+__global__ void k_take_rows(T* out, const double* Ad, const int* rows, int K) {
+  const int o = blockIdx.x * blockDim.x + threadIdx.x;
+  if (o < K) out[(size_t)blockIdx.y * K + o] = (T)Ad[(size_t)rows[blockIdx.y] * K + o];
 }
 
 // Upper triangle of V as real rows: pair t = (m, m') with m <= m' gives
@@ -276,32 +284,11 @@ __device__ __forceinline__ void put_tf32_d(float* hi, float* lo, size_t i, doubl
   lo[i] = l;
 }
 
-// A of the k-space class: the real rows of k_build_wr as TF32 pairs [Mp][Kp]
-// (zero for o >= K; rows >= 2T are zeroed beforehand), and the same rows in
-// FP64 (Ad [2T][K]) for the row sums.
-__global__ void k_build_wr_tc(float* Ah, float* Al, double* Ad, const double2* U, const double2* Phi,
-                              const int* members, const int2* tri, int K, int Kp, int msz, int npix, double scale) {
-  const int o = blockIdx.x * blockDim.x + threadIdx.x;
-  const int t = blockIdx.y;
-  if (o >= Kp) return;
-  double re = 0.0, im = 0.0;
-  if (o < K) {
-    const int2 mp = tri[t];
-    double2 acc = make_double2(0.0, 0.0);
-    for (int q = 0; q < msz; ++q) {
-      const int k = members[(size_t)o * msz + q];
-      if (k < 0) break;
-      const double2 u = U[(size_t)mp.x * npix + k], p = Phi[(size_t)mp.y * npix + k];
-      acc.x += u.x * p.x + u.y * p.y;
-      acc.y += u.x * p.y - u.y * p.x;
-    }
-    re = acc.x * scale;
-    im = acc.y * scale;
-    Ad[(size_t)(2 * t) * K + o] = re;
-    Ad[(size_t)(2 * t + 1) * K + o] = im;
-  }
-  put_tf32_d(Ah, Al, (size_t)(2 * t) * Kp + o, re);
-  put_tf32_d(Ah, Al, (size_t)(2 * t + 1) * Kp + o, im);
+// A of the k-space class: rows rows[r] of k_build_wr's as TF32 pairs [Mw][Kp]
+// (zero for o >= K; the padding rows are zeroed beforehand)
+__global__ void k_take_rows_tc(float* Ah, float* Al, const double* Ad, const int* rows, int K, int Kp) {
+  const int o = blockIdx.x * blockDim.x + threadIdx.x, r = blockIdx.y;
+  if (o < Kp) put_tf32_d(Ah, Al, (size_t)r * Kp + o, o < K ? Ad[(size_t)rows[r] * K + o] : 0.0);
 }
 
 // A of the pixel class: the real rows of k_build_vr as TF32 pairs [Mp][Kdp]
@@ -326,11 +313,13 @@ __global__ void k_build_vr_tc(float* Ah, float* Al, double* Ad, const double2* p
 }
 
 // g[r] = sum_k Ad[r][k] in FP64, one CTA of 256 threads per row (fixed order)
-__global__ void k_rowsum(double* g, const double* Ad, int K) {
+// or of |Ad[r][k]|
+template <typename T, bool ABS = false>
+__global__ void k_rowsum(double* g, const T* Ad, int K) {
   __shared__ double red[256];
   const int r = blockIdx.x;
   double acc = 0.0;
-  for (int k = threadIdx.x; k < K; k += blockDim.x) acc += Ad[(size_t)r * K + k];
+  for (int k = threadIdx.x; k < K; k += blockDim.x) acc += ABS ? fabs((double)Ad[(size_t)r * K + k]) : (double)Ad[(size_t)r * K + k];
   red[threadIdx.x] = acc;
   __syncthreads();
   for (int w = blockDim.x / 2; w > 0; w >>= 1) {
@@ -478,31 +467,37 @@ __global__ void k_build_e_tc(float* Bh, float* Bl, const int* supp, int Kd, int 
 // H[r][c] = sum_z out[z][2c..2c+1][r] + cc[c] g[r] (cc = null: 1), then
 // P[m][m'] = X + iY and P[m'][m] = X - iY with X = H[2t], Y = H[2t+1], as
 // k_scatter_herm; disk regions get diag(DG) from the left.
-// One thread per (column c, pair t), t fastest: the reads of out are float2
-// runs along m, the writes stay inside one column's matrix.  nrep > 1 (the
+// rowmap (nullable): the row of out and g that holds real row 2t or 2t + 1, -1
+// for one that is zero and was left out.
+// One thread per (column c, pair t), t fastest: the reads of out run along m,
+// the writes stay inside one column's matrix.  nrep > 1 (the
 // pixel class of a group solve, the same for every request): the matrices of
 // column (f, q) are written for frequencies f, f + nf, ...
 template <typename PT>
 __global__ void k_scatter_herm_tc(PT* P, const float* out, int Mp, int splits, const double2* cc, const double* g,
                                   int nf, int ncols, const RegionT* regs, const int* cls_regions, int nd, int nm,
-                                  const double2* DG, const int2* tri, int T, int nrep) {
+                                  const double2* DG, const int2* tri, int T, int nrep, const int* rowmap) {
   const int ncol = nf * ncols;
   const size_t plane = (size_t)2 * ncol * Mp;
   const size_t total = (size_t)ncol * T;
   for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
     const int c = (int)(i / T), t = (int)(i % T);
     const int2 mp = tri[t];
-    const double g0 = g[2 * t], g1 = g[2 * t + 1];
+    const int r0 = rowmap ? rowmap[2 * t] : 2 * t, r1 = rowmap ? rowmap[2 * t + 1] : 2 * t + 1;
+    const double g0 = r0 < 0 ? 0.0 : g[r0], g1 = r1 < 0 ? 0.0 : g[r1];
     const int f = c / ncols, q = c % ncols;
     const int j = cls_regions[q];
     double xr = 0.0, xi = 0.0, yr = 0.0, yi = 0.0;
     for (int z = 0; z < splits; ++z) {
-      const float2 re = *reinterpret_cast<const float2*>(out + z * plane + (size_t)(2 * c) * Mp + 2 * t);
-      const float2 im = *reinterpret_cast<const float2*>(out + z * plane + (size_t)(2 * c + 1) * Mp + 2 * t);
-      xr += (double)re.x;
-      yr += (double)re.y;
-      xi += (double)im.x;
-      yi += (double)im.y;
+      const float* re = out + z * plane + (size_t)(2 * c) * Mp;
+      if (r0 >= 0) {
+        xr += (double)re[r0];
+        xi += (double)re[Mp + r0];
+      }
+      if (r1 >= 0) {
+        yr += (double)re[r1];
+        yi += (double)re[Mp + r1];
+      }
     }
     const double2 k = cc ? cc[c] : make_double2(1.0, 0.0);
     xr += k.x * g0;
@@ -702,15 +697,17 @@ __global__ void k_scatter_p(PT* P, const double2* Gm, int nf, int ncols, const R
 template <typename PT>
 __global__ void k_scatter_herm(PT* P, const double2* H, int nf, int ncols, const RegionT* regs,
                                const int* cls_regions, int nd, int nm, const double2* DG, const int2* tri, int T,
-                               int nrep) {
+                               int nrep, const int* rowmap) {
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= T) return;
   const int2 mp = tri[t];
+  const int r0 = rowmap ? rowmap[2 * t] : 2 * t, r1 = rowmap ? rowmap[2 * t + 1] : 2 * t + 1;
   const size_t N = (size_t)nf * ncols;
   for (int c = blockIdx.y; c < nf * ncols; c += gridDim.y) {
     const int f = c / ncols, q = c % ncols;
     const int j = cls_regions[q];
-    const double2 X = H[(size_t)(2 * t) * N + c], Y = H[(size_t)(2 * t + 1) * N + c];
+    const double2 X = r0 < 0 ? make_double2(0.0, 0.0) : H[(size_t)r0 * N + c];
+    const double2 Y = r1 < 0 ? make_double2(0.0, 0.0) : H[(size_t)r1 * N + c];
     double2 p1 = make_double2(X.x - Y.y, X.y + Y.x);
     double2 p2 = make_double2(X.x + Y.y, X.y - Y.x);
     if (DG && regs[j].klass == 1) {
@@ -2104,6 +2101,12 @@ struct TfCache {
   // complex64 path: upper triangle of V as real rows (k_build_vr), pair table;
   // W the same way (Wr, k_build_wr) when every mode vanishes outside the mask
   DBuf Vr, Wr, tri;
+  // The k-space class's real rows that are not zero: Rw of the 2 T, in rowmap[2 T]
+  // (-1: left out).  On a grid that the modes' symmetry maps onto itself most
+  // rows cancel over the orbits (28 Bessel modes on 51 x 51: 118 of 812 are
+  // left); everywhere the imaginary rows of equal modes do.  Mw: Rw padded to 128.
+  DBuf rowmap;
+  int Rw = 0, Mw = 0;
   int T = 0;
   bool herm_w = false;
   // tensor-core path: the real rows of both classes as TF32 hi/lo pairs [Mp][Kp],
@@ -2121,7 +2124,7 @@ static size_t tf_cache_bytes(const void* p) {
   const TfCache* c = static_cast<const TfCache*>(p);
   size_t b = 0;
   for (const DBuf* d : {&c->W, &c->V, &c->Vr, &c->Wr, &c->tri, &c->rep, &c->supp, &c->U, &c->Phi, &c->members,
-                        &c->Wh, &c->Wl, &c->Vh, &c->Vl, &c->gW, &c->gV, &c->gram, &c->KT2})
+                        &c->Wh, &c->Wl, &c->Vh, &c->Vl, &c->gW, &c->gV, &c->gram, &c->KT2, &c->rowmap})
     b += d->p ? d->n : 0;
   return b;
 }
@@ -2143,7 +2146,7 @@ static int tf_setup(bf_handle* h, bf_stack* s, bf_modes* md, int mode, TfCache**
   // disks), so gap updates of an optimiser reuse them.
   if (c.modes_id == md->id && c.mode == mode) return BF_OK;
   for (DBuf* d : {&c.W, &c.V, &c.Vr, &c.Wr, &c.tri, &c.Wh, &c.Wl, &c.Vh, &c.Vl, &c.gW, &c.gV, &c.gram,
-                  &c.KT2})
+                  &c.KT2, &c.rowmap})
     d->release();
   cudaStream_t st = h->stream();
   const int nx = s->nx, ny = s->ny, nm = md->nm;
@@ -2208,17 +2211,17 @@ static int tf_setup(bf_handle* h, bf_stack* s, bf_modes* md, int mode, TfCache**
   if (!e) e = bf::launch_line_dft(true, c.Phi.p, nm, nx, ny, 1, 0, st);
   if (e) return bf_fail(h, BF_ERR_CUDA, "mode FFTs failed");
   c.Kp = (c.K + 31) / 32 * 32;
-  if (!fp64) {
-    // Phi = FFT(mask Psi) equals U = FFT(Psi) bit for bit when no mode has a
-    // non-zero pixel outside the (0/1) mask; W is then Hermitian in the mode
-    // pair, W[m'm] = conj W[mm'], and its upper triangle determines it.
-    c.herm_w = true;
-    for (int m = 0; m < nm && c.herm_w; ++m)
-      for (size_t x = 0; x < npix; ++x)
-        if (!s->mask_full[x] && md->pat[(size_t)m * npix + x] != cd(0.0, 0.0)) {
-          c.herm_w = false;
-          break;
-        }
+  // Phi = FFT(mask Psi) equals U = FFT(Psi) bit for bit when no mode has a
+  // non-zero pixel outside the (0/1) mask; W is then Hermitian in the mode
+  // pair, W[m'm] = conj W[mm'], and its upper triangle determines it.
+  c.herm_w = true;
+  for (int m = 0; m < nm && c.herm_w; ++m)
+    for (size_t x = 0; x < npix; ++x)
+      if (!s->mask_full[x] && md->pat[(size_t)m * npix + x] != cd(0.0, 0.0)) {
+        c.herm_w = false;
+        break;
+      }
+  if (!fp64 || c.herm_w) {
     std::vector<int2> tri;
     for (int m = 0; m < nm; ++m)
       for (int mp = m; mp < nm; ++mp) tri.push_back(make_int2(m, mp));
@@ -2227,49 +2230,84 @@ static int tf_setup(bf_handle* h, bf_stack* s, bf_modes* md, int mode, TfCache**
     TCKS(c.tri.alloc(h, sizeof(int2) * tri.size()));
     TCK(cudaMemcpyAsync(c.tri.p, tri.data(), sizeof(int2) * tri.size(), cudaMemcpyHostToDevice, st));
   }
-  DBuf Ad;   // FP64 real rows of the tensor-core path, for the row sums
   {
     dim3 grid(blocks_for(c.K), nm * nm);
     const double scale = 1.0 / ((double)nx * (double)ny);
     bf::note_launch();
-    if (fp64) {
-      TCKS(c.W.alloc(h, csz * (size_t)nm * nm * c.K));
-      k_build_w<double2><<<grid, 256, 0, st>>>(c.W.as<double2>(), c.U.as<double2>(), c.Phi.as<double2>(),
-                                               c.members.as<int>(), c.K, c.msz, nm, (int)npix, scale);
-    } else if (mode == 2 && c.herm_w) {
-      const size_t n = (size_t)c.Mp * c.Kp;
-      TCKS(c.Wh.alloc(h, sizeof(float) * n));
-      TCKS(c.Wl.alloc(h, sizeof(float) * n));
-      TCK(cudaMemsetAsync(c.Wh.p, 0, sizeof(float) * n, st));
-      TCK(cudaMemsetAsync(c.Wl.p, 0, sizeof(float) * n, st));
+    if (c.herm_w) {
+      DBuf Ad, d_sum, d_rows;   // the real rows in FP64, the sums of their entries' sizes, the rows kept
       TCKS(Ad.alloc(h, sizeof(double) * 2 * (size_t)c.T * c.K));
-      k_build_wr_tc<<<dim3(blocks_for(c.Kp), c.T), 256, 0, st>>>(
-          c.Wh.as<float>(), c.Wl.as<float>(), Ad.as<double>(), c.U.as<double2>(), c.Phi.as<double2>(),
-          c.members.as<int>(), c.tri.as<int2>(), c.K, c.Kp, c.msz, (int)npix, scale);
+      k_build_wr<<<dim3(blocks_for(c.K), c.T), 256, 0, st>>>(Ad.as<double>(), c.U.as<double2>(), c.Phi.as<double2>(),
+                                                             c.members.as<int>(), c.tri.as<int2>(), c.K, c.msz,
+                                                             (int)npix, scale);
       TCK(cudaGetLastError());
-      TCKS(c.gW.alloc(h, sizeof(double) * c.Mp));
-      TCK(cudaMemsetAsync(c.gW.p, 0, sizeof(double) * c.Mp, st));
+      TCKS(d_sum.alloc(h, sizeof(double) * 2 * c.T));
       bf::note_launch();
-      k_rowsum<<<2 * c.T, 256, 0, st>>>(c.gW.as<double>(), Ad.as<double>(), c.K);
-      std::vector<float> kt2(c.K);
-      for (int o = 0; o < c.K; ++o) {
-        const double kx = s->kX[c.rep_h[o].x], ky = s->kY[c.rep_h[o].y];
-        kt2[o] = (float)(kx * kx + ky * ky);
+      k_rowsum<double, true><<<2 * c.T, 256, 0, st>>>(d_sum.as<double>(), Ad.as<double>(), c.K);
+      TCK(cudaGetLastError());
+      std::vector<double> sum(2 * c.T);
+      TCK(cudaMemcpyAsync(sum.data(), d_sum.p, sizeof(double) * sum.size(), cudaMemcpyDeviceToHost, st));
+      TCK(cudaStreamSynchronize(st));
+      // A row's product with the phasors (at most 1) is at most its sum of sizes.  Zero is what four units in the
+      // last place of the largest row could not show: rows that cancel by symmetry sum to 0.2 to 1 of them, the
+      // least of the others to 1e14.
+      const double zero = 4 * DBL_EPSILON * *std::max_element(sum.begin(), sum.end());
+      std::vector<int> rows, map(2 * c.T, -1);
+      for (int r = 0; r < 2 * c.T; ++r)
+        if (!(sum[r] <= zero) || rows.empty()) {
+          map[r] = (int)rows.size();
+          rows.push_back(r);
+        }
+      c.Rw = (int)rows.size();
+      c.Mw = (c.Rw + 127) / 128 * 128;
+      TCKS(c.rowmap.alloc(h, sizeof(int) * map.size()));
+      TCK(cudaMemcpyAsync(c.rowmap.p, map.data(), sizeof(int) * map.size(), cudaMemcpyHostToDevice, st));
+      TCKS(d_rows.alloc(h, sizeof(int) * rows.size()));
+      TCK(cudaMemcpyAsync(d_rows.p, rows.data(), sizeof(int) * rows.size(), cudaMemcpyHostToDevice, st));
+      bf::note_launch();
+      const dim3 take(blocks_for(c.K), c.Rw);
+      if (fp64) {
+        TCKS(c.Wr.alloc(h, sizeof(double) * (size_t)c.Rw * c.K));
+        k_take_rows<<<take, 256, 0, st>>>(c.Wr.as<double>(), Ad.as<double>(), d_rows.as<int>(), c.K);
+      } else if (mode == 1) {
+        TCKS(c.Wr.alloc(h, sizeof(float) * (size_t)c.Rw * c.K));
+        k_take_rows<<<take, 256, 0, st>>>(c.Wr.as<float>(), Ad.as<double>(), d_rows.as<int>(), c.K);
+      } else {
+        const size_t n = (size_t)c.Mw * c.Kp;
+        TCKS(c.Wh.alloc(h, sizeof(float) * n));
+        TCKS(c.Wl.alloc(h, sizeof(float) * n));
+        TCK(cudaMemsetAsync(c.Wh.p, 0, sizeof(float) * n, st));
+        TCK(cudaMemsetAsync(c.Wl.p, 0, sizeof(float) * n, st));
+        k_take_rows_tc<<<dim3(blocks_for(c.Kp), c.Rw), 256, 0, st>>>(c.Wh.as<float>(), c.Wl.as<float>(),
+                                                                    Ad.as<double>(), d_rows.as<int>(), c.K, c.Kp);
+        TCK(cudaGetLastError());
+        DBuf g;   // of all rows, then of those kept
+        TCKS(g.alloc(h, sizeof(double) * 2 * c.T));
+        TCKS(c.gW.alloc(h, sizeof(double) * c.Rw));
+        bf::note_launch();
+        k_rowsum<<<2 * c.T, 256, 0, st>>>(g.as<double>(), Ad.as<double>(), c.K);
+        TCK(cudaGetLastError());
+        bf::note_launch();
+        k_take_rows<<<dim3(1, c.Rw), 32, 0, st>>>(c.gW.as<double>(), g.as<double>(), d_rows.as<int>(), 1);
+        std::vector<float> kt2(c.K);
+        for (int o = 0; o < c.K; ++o) {
+          const double kx = s->kX[c.rep_h[o].x], ky = s->kY[c.rep_h[o].y];
+          kt2[o] = (float)(kx * kx + ky * ky);
+        }
+        TCKS(c.KT2.alloc(h, sizeof(float) * c.K));
+        TCK(cudaMemcpyAsync(c.KT2.p, kt2.data(), sizeof(float) * c.K, cudaMemcpyHostToDevice, st));
+        TCK(cudaStreamSynchronize(st));   // kt2 is a local host array
       }
-      TCKS(c.KT2.alloc(h, sizeof(float) * c.K));
-      TCK(cudaMemcpyAsync(c.KT2.p, kt2.data(), sizeof(float) * c.K, cudaMemcpyHostToDevice, st));
-      TCK(cudaStreamSynchronize(st));   // kt2 is a local host array
-    } else if (c.herm_w) {
-      TCKS(c.Wr.alloc(h, sizeof(float) * 2 * (size_t)c.T * c.K));
-      k_build_wr<<<dim3(blocks_for(c.K), c.T), 256, 0, st>>>(c.Wr.as<float>(), c.U.as<double2>(),
-                                                              c.Phi.as<double2>(), c.members.as<int>(),
-                                                              c.tri.as<int2>(), c.K, c.msz, (int)npix, scale);
     } else {
-      // modes reaching beyond the mask (W not Hermitian): complex64 W for the
-      // SIMT GEMM (also on the tensor-core path)
+      // modes reaching beyond the mask (W not Hermitian): the complex W for the
+      // SIMT GEMMs (also on the tensor-core path)
       TCKS(c.W.alloc(h, csz * (size_t)nm * nm * c.K));
-      k_build_w<float2><<<grid, 256, 0, st>>>(c.W.as<float2>(), c.U.as<double2>(), c.Phi.as<double2>(),
-                                              c.members.as<int>(), c.K, c.msz, nm, (int)npix, scale);
+      if (fp64)
+        k_build_w<double2><<<grid, 256, 0, st>>>(c.W.as<double2>(), c.U.as<double2>(), c.Phi.as<double2>(),
+                                                 c.members.as<int>(), c.K, c.msz, nm, (int)npix, scale);
+      else
+        k_build_w<float2><<<grid, 256, 0, st>>>(c.W.as<float2>(), c.U.as<double2>(), c.Phi.as<double2>(),
+                                                c.members.as<int>(), c.K, c.msz, nm, (int)npix, scale);
     }
     TCK(cudaGetLastError());
   }
@@ -2406,6 +2444,17 @@ static int launch_gemm(bf_handle* h, const S* A, const S* B, double2* Cm, int R,
       bf::k_sum_planes<<<blocks_for(n), 256, 0, h->stream()>>>(Cm, part.as<double2>(), n, splits);
     }
   }
+  gemm_ev_end(h);
+  TCK(cudaGetLastError());
+  return BF_OK;
+}
+
+// The FP64 path's: H = A * B with real FP64 rows.
+static int launch_rgemm(bf_handle* h, const double* A, const double2* B, double2* Hm, int R, int K, int N) {
+  g_tf_gemm_flops += 4.0 * (double)R * (double)K * (double)N;
+  bf::note_launch();
+  gemm_ev_begin(h);
+  bf::k_rcgemm_d<<<dim3((N + 15) / 16, (R + 31) / 32), 128, 0, h->stream()>>>(A, B, Hm, R, K, N);
   gemm_ev_end(h);
   TCK(cudaGetLastError());
   return BF_OK;
@@ -2597,10 +2646,10 @@ static int tf_propagation_matrices(bf_handle* h, bf_stack* s, bf_modes* md, TfCa
     TCK(cudaMemcpyAsync(d_eps.p, eps_list.data(), sizeof(double2) * neps, cudaMemcpyHostToDevice, st));
     TCKS(d_peps.alloc(h, sizeof(int) * npar));
     TCK(cudaMemcpyAsync(d_peps.p, par_eps.data(), sizeof(int) * npar, cudaMemcpyHostToDevice, st));
-    const bool herm = mode == 1 && c.herm_w;   // real rows of W's upper triangle
+    const bool herm = mode != 2 && c.herm_w;   // real rows of W's upper triangle
     const bool tc = mode == 2 && c.herm_w;     // the same rows on the tensor cores
     if (!tc) {
-      TCKS(G.alloc(h, sizeof(C) * (size_t)(herm ? 2 * c.T : nm * nm) * ncol));
+      TCKS(G.alloc(h, sizeof(C) * (size_t)(herm ? c.Rw : nm * nm) * ncol));
       TCKS(KZ.alloc(h, sizeof(double2) * (size_t)neps * c.K * nf));
       bf::note_launch();
       k_build_kz<<<dim3(blocks_for(c.K), std::min(nf, 65535), neps), 256, 0, st>>>(
@@ -2615,7 +2664,9 @@ static int tf_propagation_matrices(bf_handle* h, bf_stack* s, bf_modes* md, TfCa
       TCK(cudaGetLastError());
       if (herm) {
         if constexpr (std::is_same<S, float2>::value)
-          TCKS(launch_rgemm(h, c.Wr.as<float>(), D.as<float2>(), G.as<C>(), 2 * c.T, c.K, ncol));
+          TCKS(launch_rgemm(h, c.Wr.as<float>(), D.as<float2>(), G.as<C>(), c.Rw, c.K, ncol));
+        else
+          TCKS(launch_rgemm(h, c.Wr.as<double>(), D.as<double2>(), G.as<C>(), c.Rw, c.K, ncol));
       } else {
         TCKS(launch_gemm<S>(h, c.W.as<S>(), D.as<S>(), G.as<C>(), nm * nm, c.K, ncol));
       }
@@ -2642,13 +2693,13 @@ static int tf_propagation_matrices(bf_handle* h, bf_stack* s, bf_modes* md, TfCa
           Bh.as<float>(), Bl.as<float>(), DKZ.as<float2>(), col.as<ColTC>(), c.K, c.Kp, ncol);
       TCK(cudaGetLastError());
       int splits = 1;
-      TCKS(tc_class_gemm(h, c.Wh.as<float>(), c.Wl.as<float>(), c.Mp, c.Kp, Bh.as<float>(), Bl.as<float>(),
+      TCKS(tc_class_gemm(h, c.Wh.as<float>(), c.Wl.as<float>(), c.Mw, c.Kp, Bh.as<float>(), Bl.as<float>(),
                          2 * ncol, out, &splits, tc_err));
       bf::note_launch();
       const unsigned gs = (unsigned)std::min<size_t>(blocks_for((size_t)ncol * c.T), 1u << 20);
-      k_scatter_herm_tc<S><<<gs, 256, 0, st>>>(P.as<S>(), out.as<float>(), c.Mp, splits, C0.as<double2>(),
+      k_scatter_herm_tc<S><<<gs, 256, 0, st>>>(P.as<S>(), out.as<float>(), c.Mw, splits, C0.as<double2>(),
                                                c.gW.as<double>(), nreq * nf, npar, dr, lst.as<int>(), nd, nm,
-                                               nullptr, c.tri.as<int2>(), c.T, 1);
+                                               nullptr, c.tri.as<int2>(), c.T, 1, c.rowmap.as<int>());
       TCK(cudaGetLastError());
     }
     if (!tc) {
@@ -2656,7 +2707,7 @@ static int tf_propagation_matrices(bf_handle* h, bf_stack* s, bf_modes* md, TfCa
       if (herm) {
         dim3 gs(blocks_for(c.T), std::min(ncol, 65535));
         k_scatter_herm<S><<<gs, 256, 0, st>>>(P.as<S>(), G.as<C>(), nreq * nf, npar, dr, lst.as<int>(), nd, nm,
-                                              nullptr, c.tri.as<int2>(), c.T, 1);
+                                              nullptr, c.tri.as<int2>(), c.T, 1, c.rowmap.as<int>());
       } else {
         dim3 gs(blocks_for((size_t)nm * nm), std::min(ncol, 65535));
         k_scatter_p<S><<<gs, 256, 0, st>>>(P.as<S>(), G.as<C>(), nreq * nf, npar, dr, lst.as<int>(), nd, nm, nullptr,
@@ -2737,7 +2788,7 @@ static int tf_propagation_matrices(bf_handle* h, bf_stack* s, bf_modes* md, TfCa
       const unsigned gs = (unsigned)std::min<size_t>(blocks_for((size_t)ncol * c.T), 1u << 20);
       k_scatter_herm_tc<S><<<gs, 256, 0, st>>>(P.as<S>(), out.as<float>(), c.Mp, splits, nullptr, c.gV.as<double>(),
                                                nf, npx, dr, lst.as<int>(), nd, nm, DG.as<double2>(),
-                                               c.tri.as<int2>(), c.T, nreq);
+                                               c.tri.as<int2>(), c.T, nreq, nullptr);
       TCK(cudaGetLastError());
     }
     if (mode != 2) {
@@ -2745,7 +2796,7 @@ static int tf_propagation_matrices(bf_handle* h, bf_stack* s, bf_modes* md, TfCa
       if (mode == 1) {
         dim3 gs(blocks_for(c.T), std::min(ncol, 65535));
         k_scatter_herm<S><<<gs, 256, 0, st>>>(P.as<S>(), G.as<C>(), nf, npx, dr, lst.as<int>(), nd, nm,
-                                              DG.as<double2>(), c.tri.as<int2>(), c.T, nreq);
+                                              DG.as<double2>(), c.tri.as<int2>(), c.T, nreq, nullptr);
       } else {
         dim3 gs(blocks_for((size_t)nm * nm), std::min(ncol, 65535));
         k_scatter_p<S><<<gs, 256, 0, st>>>(P.as<S>(), G.as<C>(), nf, npx, dr, lst.as<int>(), nd, nm,
