@@ -107,6 +107,20 @@ bool tc_gemm_fills_gpu(int M, int N);
 int tc_gemm_splits(int M, int N, int Kp);
 bool tc_gemm_available();
 
+// A column of the k-space class's operand: c0 = exp(-i kz0 dz), kz0, k0^2, dz and
+// the row of its (permittivity, frequency) in the table of kz - kz0.
+struct PhaseCol {
+  float2 c0, kz0, k0sq;
+  float dz;
+  int ef;
+};
+// tc_gemm_tf32x3 with M = 128 and the 2 ncol rows of B made inside the kernel:
+// Re and Im of c0 (exp(-i (kz - kz0) dz) - 1), kz - kz0 = dkz[ef][k] with rows of
+// Kp entries (zero past the last k), |(kz - kz0) dz| at most 80.  out[splits][2 ncol][128].
+int tc_phase_gemm(const float* Ahi, const float* Alo, const float2* dkz, const PhaseCol* cols, int ncol, int Kp,
+                  int splits, float* out, int* d_err, cudaStream_t st, int max_ctas);
+int tc_phase_splits(int ncol, int Kp);
+
 // ---- phasor / tilt tables (FP64 phase arguments) -----------------------
 struct RegionGeo {
   double dz;

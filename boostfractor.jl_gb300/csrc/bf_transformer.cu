@@ -334,12 +334,8 @@ __global__ void k_rowsum(double* g, const T* Ad, int K) {
 // operand builder: c0 = exp(-i kz0 dz) with kz0 = sqrt(k0^2) (the phasor's
 // transverse-momentum-zero wavenumber) in FP64 (C0, also added back by the
 // scatter), and complex64 copies of c0, kz0, k0^2 and dz (col).
-struct ColTC {
-  float2 c0, kz0, k0sq;
-  float dz;
-  int ef;   // row of the column's (permittivity, frequency) in DKZ
-};
-__global__ void k_build_c0(double2* C0, ColTC* col, const double* freqs, int nf, int ncol, int nd,
+using bf::PhaseCol;
+__global__ void k_build_c0(double2* C0, PhaseCol* col, const double* freqs, int nf, int ncol, int nd,
                            const double2* eps, const RegionT* regs, const int* par_regions, const int* par_eps,
                            int npar) {
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
@@ -352,7 +348,7 @@ __global__ void k_build_c0(double2* C0, ColTC* col, const double* freqs, int nf,
   const double dz = regs[(size_t)r * nd + par_regions[p]].dz;
   const double2 c0 = dexp_c(kz0.y * dz, -kz0.x * dz);
   C0[c] = c0;
-  ColTC q;
+  PhaseCol q;
   q.c0 = make_float2((float)c0.x, (float)c0.y);
   q.kz0 = make_float2((float)kz0.x, (float)kz0.y);
   q.k0sq = make_float2((float)k0sq.x, (float)k0sq.y);
@@ -387,35 +383,48 @@ __device__ __forceinline__ float2 cexpm1_ff(float re, float im) {
 // DKZ[e][f][o] = kz - kz0 = -kt^2 / (kz + kz0) in FP32 for the distinct
 // permittivities e of the k-space regions, once per (frequency, orbit): it has
 // no cancellation, so FP32 carries it to ~1e-7 of its own size.  KT2[o] =
-// kx^2 + ky^2 at the orbit representative.
-__global__ void k_build_dkz(float2* DKZ, const float* KT2, int K, const double* freqs, int nf, const double2* eps) {
+// kx^2 + ky^2 at the orbit representative; zero for K <= o < Kp.  A CTA's
+// wavenumbers in FP64 once, by one warp: in every thread they kept the FP64 pipe
+// busy (256 frequencies, 2080 orbits: 53 -> 12 us).
+__global__ void k_build_dkz(float2* DKZ, const float* KT2, int K, int Kp, const double* freqs, int nf,
+                            const double2* eps) {
+  __shared__ float4 kk;   // kz0, k0^2
   const int o = blockIdx.x * blockDim.x + threadIdx.x;
-  if (o >= K) return;
   const int e = blockIdx.z;
-  const float kt2 = KT2[o];
+  const float kt2 = o < K ? KT2[o] : 0.f;
   for (int f = blockIdx.y; f < nf; f += gridDim.y) {
-    const double2 k0 = k0_c(kC / freqs[f], eps[e].x, eps[e].y);
-    const double2 k0sq = make_double2(k0.x * k0.x - k0.y * k0.y, k0.x * k0.y + k0.y * k0.x);
-    const double2 kz0d = dsqrt_c(k0sq.x, k0sq.y);
-    const float2 kz0 = make_float2((float)kz0d.x, (float)kz0d.y);
-    const float2 kz = fsqrt_c((float)k0sq.x - kt2, (float)k0sq.y);
-    const float2 den = make_float2(kz.x + kz0.x, kz.y + kz0.y);
-    const float dn = den.x * den.x + den.y * den.y;
-    DKZ[((size_t)e * nf + f) * K + o] = make_float2(-kt2 * den.x / dn, kt2 * den.y / dn);   // -kt2 / den
+    if (threadIdx.x < 32) {
+      const double2 k0 = k0_c(kC / freqs[f], eps[e].x, eps[e].y);
+      const double2 k0sq = make_double2(k0.x * k0.x - k0.y * k0.y, k0.x * k0.y + k0.y * k0.x);
+      const double2 kz0d = dsqrt_c(k0sq.x, k0sq.y);
+      if (threadIdx.x == 0) kk = make_float4((float)kz0d.x, (float)kz0d.y, (float)k0sq.x, (float)k0sq.y);
+    }
+    __syncthreads();
+    const float4 q = kk;
+    __syncthreads();
+    if (o >= Kp) continue;
+    float2 v = make_float2(0.f, 0.f);
+    if (o < K) {
+      const float2 kz = fsqrt_c(q.z - kt2, q.w);
+      const float2 den = make_float2(kz.x + q.x, kz.y + q.y);
+      const float dn = den.x * den.x + den.y * den.y;
+      v = make_float2(-kt2 * den.x / dn, kt2 * den.y / dn);   // -kt2 / den
+    }
+    DKZ[((size_t)e * nf + f) * Kp + o] = v;
   }
 }
 
 // B^T of the k-space class: rows 2c, 2c + 1 = Re, Im of D[o][c] - c0[c] =
 // c0 (exp(-i (kz - kz0) dz) - 1) as TF32 pairs [2 ncol][Kp], zero for o >= K;
 // kz - kz0 from DKZ, the phase (kz - kz0) dz is a few radians at most.
-__global__ void k_build_d_tc(float* Bh, float* Bl, const float2* DKZ, const ColTC* col, int K, int Kp, int ncol) {
+__global__ void k_build_d_tc(float* Bh, float* Bl, const float2* DKZ, const PhaseCol* col, int K, int Kp, int ncol) {
   const int o = blockIdx.x * blockDim.x + threadIdx.x;
   if (o >= Kp) return;
   for (int c = blockIdx.y; c < ncol; c += gridDim.y) {
     float2 v = make_float2(0.f, 0.f);
     if (o < K) {
-      const ColTC q = col[c];
-      const float2 dkz = DKZ[(size_t)q.ef * K + o];
+      const PhaseCol q = col[c];
+      const float2 dkz = DKZ[(size_t)q.ef * Kp + o];
       const float2 m1 = cexpm1_ff(dkz.y * q.dz, -dkz.x * q.dz);
       v = make_float2(q.c0.x * m1.x - q.c0.y * m1.y, q.c0.x * m1.y + q.c0.y * m1.x);
     }
@@ -2115,6 +2124,7 @@ struct TfCache {
   DBuf Wh, Wl, Vh, Vl, gW, gV;
   DBuf gram;  // the modes' Gram matrix over the support pixels [nm][nm] (FP64)
   DBuf KT2;   // kx^2 + ky^2 at each orbit representative (FP32)
+  double kt_max = 0.0;   // its largest root
   int Kp = 0, Kdp = 0, Mp = 0;
   std::vector<int2> rep_h;
 };
@@ -2293,6 +2303,7 @@ static int tf_setup(bf_handle* h, bf_stack* s, bf_modes* md, int mode, TfCache**
         for (int o = 0; o < c.K; ++o) {
           const double kx = s->kX[c.rep_h[o].x], ky = s->kY[c.rep_h[o].y];
           kt2[o] = (float)(kx * kx + ky * ky);
+          c.kt_max = std::max(c.kt_max, std::sqrt(kx * kx + ky * ky));
         }
         TCKS(c.KT2.alloc(h, sizeof(float) * c.K));
         TCK(cudaMemcpyAsync(c.KT2.p, kt2.data(), sizeof(float) * c.K, cudaMemcpyHostToDevice, st));
@@ -2673,28 +2684,50 @@ static int tf_propagation_matrices(bf_handle* h, bf_stack* s, bf_modes* md, TfCa
     } else {
       DBuf C0, col, Bh, Bl, out;
       TCKS(C0.alloc(h, sizeof(double2) * ncol));
-      TCKS(col.alloc(h, sizeof(ColTC) * ncol));
+      TCKS(col.alloc(h, sizeof(PhaseCol) * ncol));
       bf::note_launch();
-      k_build_c0<<<blocks_for(ncol), 256, 0, st>>>(C0.as<double2>(), col.as<ColTC>(), d_freq.as<double>(), nf,
+      k_build_c0<<<blocks_for(ncol), 256, 0, st>>>(C0.as<double2>(), col.as<PhaseCol>(), d_freq.as<double>(), nf,
                                                    ncol, nd, d_eps.as<double2>(), dr, lst.as<int>(),
                                                    d_peps.as<int>(), npar);
       TCK(cudaGetLastError());
       DBuf DKZ;
-      TCKS(DKZ.alloc(h, sizeof(float2) * (size_t)neps * nf * c.K));
+      TCKS(DKZ.alloc(h, sizeof(float2) * (size_t)neps * nf * c.Kp));
       bf::note_launch();
-      k_build_dkz<<<dim3(blocks_for(c.K), std::min(nf, 65535), neps), 256, 0, st>>>(
-          DKZ.as<float2>(), c.KT2.as<float>(), c.K, d_freq.as<double>(), nf, d_eps.as<double2>());
-      TCK(cudaGetLastError());
-      const size_t nb = (size_t)2 * ncol * c.Kp;
-      TCKS(Bh.alloc(h, sizeof(float) * nb));
-      TCKS(Bl.alloc(h, sizeof(float) * nb));
-      bf::note_launch();
-      k_build_d_tc<<<dim3(blocks_for(c.Kp), std::min(ncol, 65535)), 256, 0, st>>>(
-          Bh.as<float>(), Bl.as<float>(), DKZ.as<float2>(), col.as<ColTC>(), c.K, c.Kp, ncol);
+      k_build_dkz<<<dim3(blocks_for(c.Kp), std::min(nf, 65535), neps), 256, 0, st>>>(
+          DKZ.as<float2>(), c.KT2.as<float>(), c.K, c.Kp, d_freq.as<double>(), nf, d_eps.as<double2>());
       TCK(cudaGetLastError());
       int splits = 1;
-      TCKS(tc_class_gemm(h, c.Wh.as<float>(), c.Wl.as<float>(), c.Mw, c.Kp, Bh.as<float>(), Bl.as<float>(),
+      // One tile of rows (up to 11 modes, more where most rows are zero) makes B as it goes; with more tiles a B made
+      // once and stored serves them all.  8 modes, 21 regions, 256 frequencies: 72 us against 114 us, a group
+      // of 16 663 us against 1359 us (and 2.9 GB less of workspace).
+      // Its sine wants |(kz - kz0) dz| <= 80 (6 cm of air at 20 GHz).
+      double most = 0.0;
+      for (const double2& e : eps_list) most = std::max(most, std::sqrt(std::hypot(e.x, e.y)));
+      most = 2 * (2 * M_PI / kC) * most * *std::max_element(freqs.begin(), freqs.begin() + nf) + c.kt_max;
+      double far = 0.0;
+      for (int r = 0; r < nreq; ++r)
+        for (int j : kreg) far = std::max(far, std::fabs(regs[(size_t)r * nd + j].dz));
+      if (c.Mw == 128 && most * far <= 80.0) {
+        splits = bf::tc_phase_splits(ncol, c.Kp);
+        TCKS(out.alloc(h, sizeof(float) * (size_t)splits * 2 * ncol * c.Mw));
+        g_tf_gemm_flops += 3.0 * 2.0 * (double)c.Mw * (double)c.Kp * 2.0 * (double)ncol;
+        gemm_ev_begin(h);
+        const int e = bf::tc_phase_gemm(c.Wh.as<float>(), c.Wl.as<float>(), DKZ.as<float2>(), col.as<PhaseCol>(), ncol,
+                                        c.Kp, splits, out.as<float>(), tc_err, st, h->sm_cap);
+        gemm_ev_end(h);
+        if (e)
+          return bf_fail(h, BF_ERR_CUDA, std::string("tensor-core GEMM: ") + cudaGetErrorString((cudaError_t)e));
+      } else {
+        const size_t nb = (size_t)2 * ncol * c.Kp;
+        TCKS(Bh.alloc(h, sizeof(float) * nb));
+        TCKS(Bl.alloc(h, sizeof(float) * nb));
+        bf::note_launch();
+        k_build_d_tc<<<dim3(blocks_for(c.Kp), std::min(ncol, 65535)), 256, 0, st>>>(
+            Bh.as<float>(), Bl.as<float>(), DKZ.as<float2>(), col.as<PhaseCol>(), c.K, c.Kp, ncol);
+        TCK(cudaGetLastError());
+        TCKS(tc_class_gemm(h, c.Wh.as<float>(), c.Wl.as<float>(), c.Mw, c.Kp, Bh.as<float>(), Bl.as<float>(),
                          2 * ncol, out, &splits, tc_err));
+      }
       bf::note_launch();
       const unsigned gs = (unsigned)std::min<size_t>(blocks_for((size_t)ncol * c.T), 1u << 20);
       k_scatter_herm_tc<S><<<gs, 256, 0, st>>>(P.as<S>(), out.as<float>(), c.Mw, splits, C0.as<double2>(),
