@@ -498,7 +498,7 @@ size_t bf_stack_device_bytes(const bf_stack* s) {
   if (s->d_surf) b += sizeof(double2) * s->nd * npix;
   if (const Workspace* w = s->ws) {
     for (const DBuf* d : {&w->freq, &w->reg, &w->phasor, &w->tab_idx, &w->compact_A, &w->tidx, &w->tregs, &w->tilt, &w->init, &w->state,
-                          &w->add, &w->coef, &w->exitacc, &w->steps, &w->tmp, &w->beta, &w->mg, &w->exit_full[0],
+                          &w->add, &w->coef, &w->exitacc, &w->steps, &w->run, &w->tmp, &w->beta, &w->mg, &w->exit_full[0],
                           &w->exit_full[1], &w->direct[0], &w->direct[1]})
       b += dbuf_bytes(*d);
   }
@@ -1234,6 +1234,10 @@ static int run_fused(bf_handle* h, bf_stack* s, const std::string& key,
       all.insert(all.end(), sv.begin(), sv.end());
     }
     CKS(upload(h, w.steps, all.data(), sizeof(StepDesc) * all.size()));
+    std::vector<int> run = {0, 0};   // the barrier words of a run of stages, then the stages' first steps
+    for (size_t o : w.stage_off) run.push_back((int)o);
+    run.push_back((int)all.size());
+    CKS(upload(h, w.run, run.data(), sizeof(int) * run.size()));
     w.has_direct.assign(p.nexit, 0);
     for (int k = 0; k < p.nexit; ++k)
       if (!p.exit_direct[k].empty()) {
@@ -1324,11 +1328,26 @@ static int run_fused(bf_handle* h, bf_stack* s, const std::string& key,
   prof_mark(h, 1);
   const unsigned long long l1 = bf::launch_count();
   auto run_stages = [&]() -> int {
-    for (size_t k = 0; k < w.stage_off.size(); ++k) {
+    auto in_run = [&](size_t k) {
+      return fp64 && a.mg && w.stage_len[k] > 0 && bf::split_stage((int)w.stage_len[k], nf) &&
+             bf::split_run_fits(N, (int)w.stage_len[k], nf);
+    };
+    for (size_t k = 0, next; k < w.stage_off.size(); k = next) {
+      size_t len = w.stage_len[k];
+      for (next = k + 1; in_run(k) && next < w.stage_off.size() && in_run(next); ++next)
+        len = std::max(len, w.stage_len[next]);
       a.steps = w.steps.as<StepDesc>() + w.stage_off[k];
+      a.run_len = 0;
+      if (next > k + 1) {
+        a.steps = w.steps.as<StepDesc>();
+        a.run_tab = w.run.as<int>() + 2 + k;
+        a.run_bar = w.run.as<unsigned>();
+        a.run_len = (int)(next - k);
+        a.max_ctas = h->sm_cap;
+      }
       int e;
-      if (fp64) e = bf::launch_fused_stage_d(N, *reinterpret_cast<bf::FusedArgs<double2>*>(&a), (int)w.stage_len[k], st);
-      else e = bf::launch_fused_stage_f(N, *reinterpret_cast<bf::FusedArgs<float2>*>(&a), (int)w.stage_len[k], st);
+      if (fp64) e = bf::launch_fused_stage_d(N, *reinterpret_cast<bf::FusedArgs<double2>*>(&a), (int)len, st);
+      else e = bf::launch_fused_stage_f(N, *reinterpret_cast<bf::FusedArgs<float2>*>(&a), (int)len, st);
       if (e) return fail(h, BF_ERR_CUDA, std::string("fused stage: ") + cudaGetErrorString((cudaError_t)e));
     }
     return BF_OK;
@@ -1341,8 +1360,8 @@ static int run_fused(bf_handle* h, bf_stack* s, const std::string& key,
   std::string gkey = key + (fp64 ? "|d" : "|f");
   {
     const void* ptrs[] = {a.state, a.phasor, a.tilt, a.tilt_idx, a.mask, a.coefs, a.exitacc, a.addbuf,
-                          a.err, w.steps.p, a.mg, a.tab_idx};
-    const long long ints[] = {nf, a.nbx, a.nby, a.nslots, a.ntab, a.fold, a.ntilt, N, (long long)fp64,
+                          a.err, w.steps.p, a.mg, a.tab_idx, w.run.p};
+    const long long ints[] = {h->sm_cap, nf, a.nbx, a.nby, a.nslots, a.ntab, a.fold, a.ntilt, N, (long long)fp64,
                               (long long)w.stage_off.size(), h->device, a.variant};
     gkey.append(reinterpret_cast<const char*>(ptrs), sizeof(ptrs));
     gkey.append(reinterpret_cast<const char*>(ints), sizeof(ints));

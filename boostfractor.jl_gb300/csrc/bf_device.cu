@@ -140,6 +140,15 @@ size_t split_tile_bytes(int N, int nby, int nfreq, int nsteps, bool fp64) {
 // Whether a stage of `nsteps` steps x `nfreq` frequencies takes the split path.
 bool split_stage(int nsteps, int nfreq) { return (long long)nsteps * nfreq < sm_count(); }
 
+// One launch for a run of split stages while a phase has at most 4 warps an SM: above, the phases are bound by the FP64
+// pipe, and larger CTAs in separate launches are as fast (dancer at 64^2, 31 stages: 1 frequency 1.20 -> 1.13 ms, 4
+// 2.13 -> 1.20 ms; 5 and more take the launches).  complex64, which has no such pipe, stays with the launches (0.65
+// against 0.75 ms).
+bool split_run_fits(int N, int nsteps, int nfreq) {
+  const int lanes = N == 40 || N == 80 || N == 160 ? 4 : N >= 256 ? 16 : 8;   // a line's threads, at least
+  return (long long)nsteps * nfreq * 2 * N * lanes / 32 <= 4LL * sm_count();
+}
+
 static size_t smem_for(int N, int nby, size_t csz) {
   switch (N) {
     case 8: return fused_smem_for<8>(nby, csz);

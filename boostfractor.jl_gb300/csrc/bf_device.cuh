@@ -48,6 +48,13 @@ struct FusedArgs {
   int* err;                       // set to 1 if a bounded wait gave up
   C* mg;                          // row tiles of the split-phase path [step][f][2][nby][N+2], or null
   int variant;                    // host side: fused-kernel variant (FusedVariant), 0 = by rule
+  // a run of split-phase stages in one launch: stage k's steps are
+  // steps[run_tab[k] .. run_tab[k + 1]); run_bar: the grid barrier's count and
+  // its abort flag, zeroed by the launch; run_len = 0: one stage, `steps`
+  const int* run_tab = nullptr;
+  unsigned* run_bar = nullptr;
+  int run_len = 0;
+  int max_ctas = 0;               // 0 = no limit on the run's CTAs
 };
 
 // Variants of the fused stage kernel for stages that do not take the
@@ -82,6 +89,8 @@ bool fused_supported(int N, int nbx, int nby, bool fp64);
 size_t split_tile_bytes(int N, int nby, int nfreq, int nsteps, bool fp64);
 bool split_stage(int nsteps, int nfreq);
 bool split_length(int N);
+// Whether consecutive split stages of at most `nsteps` steps run in one launch.
+bool split_run_fits(int N, int nsteps, int nfreq);
 
 // Shortest transform length of the fused kernel that gives the fields of a box
 // of `box` pixels exactly (the propagator's kernel truncated to the offsets

@@ -107,7 +107,7 @@ struct StageGraph {
 // Per-stack device workspace reused across solves (no allocation on the
 // steady-state path) and the cached bounce plan.
 struct Workspace {
-  DBuf freq, reg, phasor, tidx, tregs, tilt, init, state, add, coef, exitacc, steps, tmp, beta, mg;
+  DBuf freq, reg, phasor, tidx, tregs, tilt, init, state, add, coef, exitacc, steps, run, tmp, beta, mg;
   DBuf tab_idx, compact_A;       // table of each region; compact_matrix
   DBuf exit_full[2], direct[2];
   std::string plan_key;  // solver/nmax/emission of the cached plan

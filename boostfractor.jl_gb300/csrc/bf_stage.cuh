@@ -534,14 +534,15 @@ __device__ __forceinline__ void joint_phase3(const FusedArgs<C>& a, C* MA, C* MB
 // Boundary mix of a step over the box: A' = cAA A~ + cAB B~ (+ add),
 // B' = cBA A~ + cBB B~, stored masked; X~ is the propagated field (row tile)
 // of a propagated slot times its region's tilt/surface map, else the slot's
-// stored field.  Pixels i0, i0 + is, ..., K at a time: the loads of K pixels
+// stored field.  Pixels i0, i0 + is, ... below `end`, K at a time: the loads of K pixels
 // come before their stores (which may alias them, as far as the compiler
 // knows), so memory is waited for once per K pixels instead of once per pixel.
 template <typename C, int N, int K>
 __device__ __forceinline__ void joint_mix(const FusedArgs<C>& a, const StepDesc& sd, int f, const C* MA,
-                                          const C* MB, bool pa, bool pb, int i0, int is) {
+                                          const C* MB, bool pa, bool pb, int i0, int is, int end = 1 << 30) {
   constexpr int P = FusedCtx<C, N>::P;
   const int nbx = a.nbx, plane = nbx * a.nby;
+  end = min(end, plane);
   const unsigned magic = 0xffffffffu / (unsigned)nbx + 1u;   // i / nbx = umulhi(i, magic) for i < 2^16, nbx > 1
   C* stA = sd.sa >= 0 ? a.state + ((size_t)f * a.nslots + sd.sa) * plane : nullptr;
   C* stB = sd.sb >= 0 ? a.state + ((size_t)f * a.nslots + sd.sb) * plane : nullptr;
@@ -551,7 +552,7 @@ __device__ __forceinline__ void joint_mix(const FusedArgs<C>& a, const StepDesc&
   const C* tmB = tiB >= 0 ? a.tilt + ((size_t)f * a.ntilt + tiB) * plane : nullptr;
   const C* cf = a.coefs + 4 * sd.coef;
   const C cAA = cf[0], cAB = cf[1], cBA = cf[2], cBB = cf[3];
-  for (int b = i0; b < plane; b += K * is) {
+  for (int b = i0; b < end; b += K * is) {
     C tA[K], tB[K], A[K], B[K], ad[K];
     bool in[K];
 #pragma unroll
@@ -702,6 +703,104 @@ __global__ void __launch_bounds__(kSplitThreads) k_split_phase(FusedArgs<cplx_t<
   }
 }
 
+// ---- a run of split stages in one launch --------------------------------------
+// The same phases by one resident grid of single-warp CTAs (the FP64 pipe takes
+// 16 cycles a warp instruction, so a phase's warps go to as many SMs as there
+// are), with barriers in place of the launches: three a stage, since the warp
+// that transforms a row of A and B back also mixes it.  Bound by latency: the
+// one-frequency dancer at 64^2 (4 steps a stage) took 35 us a stage with four
+// launches, 29 us here, of which the barriers are 4 (1.3 us each).
+
+// Every CTA of the (cooperatively launched) grid arrives; false when the wait
+// gave up after ~2 s or another CTA's did.
+__device__ __forceinline__ bool run_barrier(unsigned* bar, unsigned target, int* err) {
+  __syncwarp();
+  bool ok = true;
+  if ((threadIdx.x & 31) == 0) {
+    __threadfence();
+    atomicAdd(bar, 1u);
+    const long long t0 = clock64();
+    for (;;) {
+      unsigned n;
+      asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(n) : "l"(bar) : "memory");
+      if (n >= target) break;
+      if (*reinterpret_cast<volatile unsigned*>(bar + 1)) {
+        ok = false;
+        break;
+      }
+      if (clock64() - t0 > 4000000000LL) {
+        atomicExch(err, 1);
+        atomicExch(bar + 1, 1u);
+        ok = false;
+        break;
+      }
+    }
+    __threadfence();
+  }
+  __syncwarp();
+  return __shfl_sync(0xffffffffu, (int)ok, 0) != 0;
+}
+
+template <typename R, int N, int NZ>
+__global__ void __launch_bounds__(32) k_split_run(FusedArgs<cplx_t<R>> a) {
+  using C = cplx_t<R>;
+  using X = FusedCtx<C, N>;
+  constexpr int G = X::G, RR = X::RR, CC = X::CC, P = X::P, NT = 32 / G;
+  constexpr int RW = NT > 1 ? NT / 2 : 1;   // rows of a warp's last phase, of A and of B
+  extern __shared__ __align__(128) unsigned char smem_raw[];
+  const int lane = threadIdx.x, team = lane / G, g = lane % G;
+  const int nbx = a.nbx, nby = a.nby;
+  C* scr = reinterpret_cast<C*>(smem_raw) + team * X::T::template scratch<false>();
+  C tw[RR];
+  team_twiddles<N>(tw, g);
+  const int z[3] = {(2 * nby + NT - 1) / NT, (2 * N + NT - 1) / NT, (nby + RW - 1) / RW};
+  unsigned target = 0;
+  for (int k = 0; k < a.run_len; ++k) {
+    const int off = a.run_tab[k], ns = a.run_tab[k + 1] - off;
+    for (int ph = 0; ph < 3; ++ph) {
+      const int total = ns * a.nfreq * z[ph];
+      for (int vb = blockIdx.x; vb < total; vb += gridDim.x) {
+        const int zi = vb % z[ph], s = vb / z[ph] % ns, f = vb / (z[ph] * ns);
+        const StepDesc sd = a.steps[off + s];
+        C* MA = a.mg + ((size_t)s * a.nfreq + f) * 2 * (size_t)nby * P;
+        C* MB = MA + (size_t)nby * P;
+        const bool pa = sd.ra >= 0, pb = sd.rb >= 0;
+        if (ph == 0) {
+          joint_phase1<C, N, NZ, NT, true>(a, sd, f, MA, MB, scr, tw, team, g, zi * NT, 2 * nby, pa, pb);
+        } else if (ph == 1) {
+          const int QW = a.fold ? N / 2 : N;
+          const C* QA = pa ? a.phasor + ((size_t)f * a.ntab + a.tab_idx[sd.ra]) * (size_t)(QW * QW) : nullptr;
+          const C* QB = pb ? a.phasor + ((size_t)f * a.ntab + a.tab_idx[sd.rb]) * (size_t)(QW * QW) : nullptr;
+          joint_phase2<C, N, NZ, NT, true>(a, QA, QB, MA, MB, scr, tw, team, g, zi * NT, 2 * N);
+        } else {
+          const int y0 = zi * RW;
+#pragma unroll
+          for (int h = 0; h < 2 * RW / NT; ++h) {
+            const int q = h * NT + team, y = y0 + q / 2;
+            const bool isb = q & 1, act = y < nby && (isb ? pb : pa);
+            C* row = (isb ? MB : MA) + (act ? y : 0) * P;
+            C v[RR];
+#pragma unroll
+            for (int j = 0; j < CC; ++j)
+#pragma unroll
+              for (int i = 0; i < G; ++i) v[j * G + i] = act ? row[g * CC + j + RR * i] : czero<C>();
+            X::T::template inverse<false>(v, tw, scr, g);
+            if (act)
+#pragma unroll
+              for (int r = 0; r < NZ; ++r)
+                if (g + G * r < nbx) row[g + G * r] = v[r];
+          }
+          __syncwarp();
+          joint_mix<C, N, 1>(a, sd, f, MA, MB, pa, pb, y0 * nbx + lane, 32, (y0 + RW) * nbx);
+        }
+      }
+      if (k + 1 == a.run_len && ph == 2) break;
+      target += gridDim.x;
+      if (!run_barrier(a.run_bar, target, a.err)) return;
+    }
+  }
+}
+
 static const size_t kMaxSmem = 227 * 1024;
 
 // Shared memory of one SM (bytes) and what the driver reserves per CTA.
@@ -722,7 +821,40 @@ static int launch_fused_v(const FusedArgs<cplx_t<R>>& a, dim3 grid, size_t smem,
 }
 
 template <typename R, int N, int NZ>
+static int launch_split_run(const FusedArgs<cplx_t<R>>& a, int nsteps, cudaStream_t st) {
+  using T = Team<N>;
+  constexpr int NT = 32 / T::G;
+  const size_t smem = sizeof(cplx_t<R>) * NT * T::template scratch<false>();
+  int dev = 0, sms = 0, per = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  if (e == cudaSuccess)
+    e = cudaFuncSetAttribute(k_split_run<R, N, NZ>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxSmem);
+  if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_split_run<R, N, NZ>, 32, smem);
+  if (e != cudaSuccess) return (int)e;
+  if (a.max_ctas > 0) sms = std::min(sms, a.max_ctas);
+  // no more CTAs than the widest phase has warps: each one more lengthens the barriers
+  const long long widest = (long long)nsteps * a.nfreq * std::max((2 * N + NT - 1) / NT, a.nby);
+  const int grid = (int)std::min<long long>(widest, (long long)sms * std::min(per, 4));
+  e = cudaMemsetAsync(a.run_bar, 0, 2 * sizeof(unsigned), st);
+  if (e != cudaSuccess) return (int)e;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeCooperative;
+  attr[0].val.cooperative = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(32);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  note_launch();
+  return (int)cudaLaunchKernelEx(&cfg, k_split_run<R, N, NZ>, a);
+}
+
+template <typename R, int N, int NZ>
 static int launch_split(const FusedArgs<cplx_t<R>>& a, int nsteps, cudaStream_t st) {
+  if (a.run_len > 0) return launch_split_run<R, N, NZ>(a, nsteps, st);
   using T = Team<N>;
   const int nteam = kSplitThreads / T::G;
   const size_t smem = sizeof(cplx_t<R>) * nteam * T::template scratch<false>();
