@@ -3548,119 +3548,78 @@ extern "C" int bf_transformer(bf_handle* h, bf_stack* s, bf_modes* md, int nf, c
 // the boundary factors carry 1/(2 n_j) and the emission carries S_j (folded on
 // the host); the phase k0 dz = pi (2 f / c) n dz goes through sincospi, whose
 // argument reduction is exact and cheap; a lossless region (real eps, held as
-// re - 0.0im, so Im n = -0.0 and exp(Im k0 dz) = 1 exactly) needs no exp, and
-// its 1/P is conj(P).
+// re - 0.0im, so Im n = -0.0 and exp(Im k0 dz) = 1 exactly) needs no exp, its
+// 1/P is conj(P), and between two of them the products with the zero imaginary
+// parts of a and b, which would add zeros, are left out (26 FP64 instructions
+// for 36); a region whose phase equals that of the region two before it (equal
+// disks between gaps) takes its sine and cosine over (the branch is the same for
+// a warp's threads, neighbouring frequencies of one configuration).
+// Which product of a sum is rounded by itself is written out (tf1d_mul, tf1d_turn,
+// and the sums of two products each rounded): stacks of many disks have localised
+// resonances with beta^2 above 1e7, which amplify a unit of rounding 1e5 to 1e7
+// times, so another order of the same formula moves beta^2 by more than 1e-9.
+// The real rotation on T21 + T22 and (T21 - T22) / n, 12 instructions a region,
+// does (1.1e-9 on one draw of spacings) and is not used.
+// Bound by the FP64 pipe (two lanes an SM and clock).  4096 configurations x 256
+// frequencies, 20 equal disks, whole call: 4.31 ms; with every region in complex
+// and a phase of its own 5.55 ms, the same bits; as rotations 2.50 ms.
 struct Region1D {
   double2 a, b;   // (n_{j-1} + n_j) / (2 n_{j-1}),  (n_{j-1} - n_j) / (2 n_{j-1})
   double2 Se;     // S_j * emit
   double2 n;      // sqrt(eps_j) of the propagated region
+  int real;       // a, b and n have no imaginary part
 };
 
-__global__ void k_tf1d(const double* dist, int nd, const Region1D* rg, const double* freqs, int nf, int nconf,
-                       double2* boost, double* beta2) {
+// x y of a boundary factor and an amplitude; x p of an amplitude and a phase
+__device__ __forceinline__ double2 tf1d_mul(double2 x, double2 y) {
+  return make_double2(fma(x.x, y.x, -__dmul_rn(x.y, y.y)), fma(x.x, y.y, __dmul_rn(x.y, y.x)));
+}
+__device__ __forceinline__ double2 tf1d_turn(double2 x, double2 p) {
+  return make_double2(fma(x.x, p.x, -__dmul_rn(x.y, p.y)), fma(x.y, p.x, __dmul_rn(x.x, p.y)));
+}
+
+__global__ void __launch_bounds__(256) k_tf1d(const double* __restrict__ dist, int nd, const Region1D* __restrict__ rg,
+                                              const double* __restrict__ freqs, int nf, int nconf, double2* boost,
+                                              double* beta2) {
   const long i = blockIdx.x * (long)blockDim.x + threadIdx.x;
   if (i >= (long)nconf * nf) return;
   const int c = (int)(i / nf), f = (int)(i % nf);
   const double* dz = dist + (size_t)c * nd;
   const double x2 = 2.0 * freqs[f] / kC;   // 2 / lambda: k0 = pi x2 n
   double2 t21 = make_double2(0.0, 0.0), t22 = make_double2(1.0, 0.0), ax = make_double2(0.0, 0.0);
-  for (int j = 1; j < nd; ++j) {
-    const Region1D g = rg[j];
-    ax = bf::cadd(ax, bf::cmul(g.Se, bf::cadd(t21, t22)));
-    double sn, cs;
-    sincospi(x2 * g.n.x * dz[j], &sn, &cs);
-    double2 P = make_double2(cs, -sn), Pi = make_double2(cs, sn);
-    if (g.n.y != 0.0) {   // uniform across the warp: every thread is at region j
-      const double m = exp(M_PI * x2 * g.n.y * dz[j]), mi = 1.0 / m;
-      P = make_double2(m * cs, -m * sn);
-      Pi = make_double2(mi * cs, mi * sn);
-    }
-    const double2 u = bf::cadd(bf::cmul(g.a, t21), bf::cmul(g.b, t22));
-    const double2 v = bf::cadd(bf::cmul(g.b, t21), bf::cmul(g.a, t22));
-    t21 = bf::cmul(u, P);
-    t22 = bf::cmul(v, Pi);
-  }
-  const double d = t22.x * t22.x + t22.y * t22.y;
-  const double2 q = make_double2(-(ax.x * t22.x + ax.y * t22.y) / d, -(ax.y * t22.x - ax.x * t22.y) / d);
-  if (boost) boost[i] = q;
-  beta2[i] = q.x * q.x + q.y * q.y;
-}
-
-// The same chain when every permittivity is real and positive, which is what a
-// scan of spacings uses.  |P| = 1 then, and on p = T21 + T22 and
-// h = (T21 - T22) / n the region's factor is the real rotation
-//   p' = cos p - i (n sin) h,   h' = cos h - i (sin / n) p,
-// and S_j meets p alone: 12 FP64 instructions instead of 26, and of the phase
-// only the sine and cosine.  A region whose phase equals that of the region two
-// before it (equal disks between gaps) takes it over; the branch is the same for
-// a warp's threads, which are neighbouring frequencies of one configuration.
-// Bound by the FP64 pipe (two lanes an SM and clock).  4096 configurations x 256
-// frequencies, 20 equal disks: 5.20 -> 2.13 ms.
-struct Region1DReal {
-  double n, inv, S;   // sqrt(eps_j), its inverse, S_j
-};
-
-// cos(pi x) and sin(pi x) for |x| < 2^50: a half turn is taken off exactly and the series of both run on at most a
-// quarter of pi, to below half a unit of the last place
-__device__ __forceinline__ void cospi_sinpi(double x, double* cs, double* sn) {
-  const double kMagic = 6755399441055744.0;   // 1.5 2^52: adding it rounds to a whole number
-  const double m = fma(x, 2.0, kMagic);
-  const int k = __double2loint(m);
-  const double r = fma(x, 2.0, -(m - kMagic)), t = r * r;   // x pi = (k + r) pi / 2
-  double c = 6.565963114979473e-11;
-  c = fma(c, t, -6.386603083791852e-09);
-  c = fma(c, t, 4.710874778818172e-07);
-  c = fma(c, t, -2.5202042373060607e-05);
-  c = fma(c, t, 0.0009192602748394266);
-  c = fma(c, t, -0.02086348076335296);
-  c = fma(c, t, 0.25366950790104803);
-  c = fma(c, t, -1.2337005501361697);
-  c = fma(c, t, 1.0);
-  double s = -6.688035109811468e-10;
-  s = fma(s, t, 5.692172921967927e-08);
-  s = fma(s, t, -3.598843235212085e-06);
-  s = fma(s, t, 0.00016044118478735983);
-  s = fma(s, t, -0.004681754135318688);
-  s = fma(s, t, 0.07969262624616705);
-  s = fma(s, t, -0.6459640975062463);
-  s = fma(s * t, r, r * 1.5707963267948966);
-  const double a = (k & 1) ? s : c, b = (k & 1) ? c : s;
-  *cs = ((k + 1) & 2) ? -a : a;
-  *sn = (k & 2) ? -b : b;
-}
-
-__global__ void __launch_bounds__(256) k_tf1d_real(const double* __restrict__ dist, int nd,
-                                                   const Region1DReal* __restrict__ rg, double inv_n0,
-                                                   const double* __restrict__ x2s, int nf, int nconf, double2 emit,
-                                                   double2* boost, double* beta2) {
-  const long i = blockIdx.x * (long)blockDim.x + threadIdx.x;
-  if (i >= (long)nconf * nf) return;
-  const int c = (int)(i / nf), f = (int)(i - (long)c * nf);
-  const double* dz = dist + (size_t)c * nd;
-  const double x2 = x2s[f];
-  double2 p = make_double2(1.0, 0.0), hh = make_double2(-inv_n0, 0.0), ax = make_double2(0.0, 0.0);
-  // sine and cosine of the last two regions, and what their phases came from
-  double cs[2] = {1.0, 1.0}, sm[2] = {0.0, 0.0}, sd[2] = {0.0, 0.0}, was[2] = {0.0, 0.0}, nwas[2] = {0.0, 0.0};
-  double n = 1.0;
+  // sine and cosine of the last two regions, and what their phases came from (no region has n = 0)
+  double cs[2] = {1.0, 1.0}, sn[2] = {0.0, 0.0}, was[2] = {0.0, 0.0}, nwas[2] = {0.0, 0.0};
   auto step = [&](int j, int q) {
-    const Region1DReal g = rg[j];
+    const Region1D& g = rg[j];
     const double d = dz[j];
-    n = g.n;
-    if (d != was[q] || g.n != nwas[q]) {
-      double sn;
-      cospi_sinpi(x2 * g.n * d, &cs[q], &sn);
-      sm[q] = sn * g.n;
-      sd[q] = sn * g.inv;
-      was[q] = d;
-      nwas[q] = g.n;
+    const double2 w = bf::cadd(t21, t22);
+    if (g.Se.y == 0.0) {
+      ax.x = __dadd_rn(ax.x, __dmul_rn(g.Se.x, w.x));
+      ax.y = __dadd_rn(ax.y, __dmul_rn(g.Se.x, w.y));
+    } else {
+      ax = bf::cadd(ax, tf1d_mul(g.Se, w));
     }
-    ax.x = fma(g.S, p.x, ax.x);
-    ax.y = fma(g.S, p.y, ax.y);
-    const double2 u = p;
-    p.x = fma(sm[q], hh.y, cs[q] * u.x);
-    p.y = fma(-sm[q], hh.x, cs[q] * u.y);
-    hh.x = fma(sd[q], u.y, cs[q] * hh.x);
-    hh.y = fma(-sd[q], u.x, cs[q] * hh.y);
+    if (d != was[q] || g.n.x != nwas[q]) {
+      sincospi(x2 * g.n.x * d, &sn[q], &cs[q]);
+      was[q] = d;
+      nwas[q] = g.n.x;
+    }
+    double2 P = make_double2(cs[q], -sn[q]), Pi = make_double2(cs[q], sn[q]), u, v;
+    if (g.real) {   // uniform across the warp: every thread is at region j
+      auto two = [](double x, double s, double y, double t) { return __dadd_rn(__dmul_rn(x, s), __dmul_rn(y, t)); };
+      u = make_double2(two(g.a.x, t21.x, g.b.x, t22.x), two(g.a.x, t21.y, g.b.x, t22.y));
+      v = make_double2(two(g.b.x, t21.x, g.a.x, t22.x), two(g.b.x, t21.y, g.a.x, t22.y));
+    } else {
+      if (g.n.y != 0.0) {
+        const double m = exp(M_PI * x2 * g.n.y * d), mi = 1.0 / m;
+        P = make_double2(m * P.x, m * P.y);
+        Pi = make_double2(mi * Pi.x, mi * Pi.y);
+      }
+      u = bf::cadd(tf1d_mul(g.a, t21), tf1d_mul(g.b, t22));
+      v = bf::cadd(tf1d_mul(g.b, t21), tf1d_mul(g.a, t22));
+    }
+    t21 = tf1d_turn(u, P);
+    t22 = tf1d_turn(v, Pi);
   };
   int j = 1;
   for (; j + 1 < nd; j += 2) {
@@ -3668,12 +3627,11 @@ __global__ void __launch_bounds__(256) k_tf1d_real(const double* __restrict__ di
     step(j + 1, 0);
   }
   if (j < nd) step(j, 1);
-  const double2 t22 = make_double2(0.5 * fma(-n, hh.x, p.x), 0.5 * fma(-n, hh.y, p.y));
-  ax = bf::cmul(emit, ax);
-  const double d = 1.0 / (t22.x * t22.x + t22.y * t22.y);
-  const double2 q = make_double2(-(ax.x * t22.x + ax.y * t22.y) * d, -(ax.y * t22.x - ax.x * t22.y) * d);
+  const double d = fma(t22.x, t22.x, __dmul_rn(t22.y, t22.y));
+  const double2 q = make_double2(-fma(ax.x, t22.x, __dmul_rn(ax.y, t22.y)) / d,
+                                 -fma(ax.y, t22.x, -__dmul_rn(ax.x, t22.y)) / d);
   if (boost) boost[i] = q;
-  beta2[i] = q.x * q.x + q.y * q.y;
+  beta2[i] = fma(q.x, q.x, __dmul_rn(q.y, q.y));
 }
 
 // Cross-request batch: the transformer for nreq stacks that differ only in
@@ -3761,51 +3719,23 @@ extern "C" int bf_transformer_1d_batch(bf_handle* h, int nconf, int nd, const do
     const cd Se = S * (emit ? cd(emit[0], emit[1]) : cd(1.0, 0.0));
     rg[j].Se = make_double2(Se.real(), Se.imag());
     rg[j].n = make_double2(nl.real(), nl.imag());
+    rg[j].real = a.imag() == 0.0 && b.imag() == 0.0 && nl.imag() == 0.0;
   }
   const size_t npts = (size_t)nconf * nf;
   DBuf d_dist, d_rg, d_f, d_b, d_b2;
   TCKS(d_dist.alloc(h, sizeof(double) * (size_t)nconf * nd));
   TCK(cudaMemcpyAsync(d_dist.p, distances, sizeof(double) * (size_t)nconf * nd, cudaMemcpyHostToDevice, st));
-  // the real chain's phases stay below cospi_sinpi's range, and n and 1/n within a square of the double's range
-  bool real = true;
-  double nmax = 0.0, dmax = 0.0, fmax = 0.0;
-  for (int j = 0; j < nd; ++j) {
-    real = real && e[j].imag() == 0.0 && e[j].real() >= 1e-40 && e[j].real() <= 1e40;
-    if (j > 0) nmax = std::max(nmax, std::sqrt(std::fabs(e[j].real())));
-  }
-  for (size_t i = 0; i < (size_t)nconf * nd; ++i) dmax = std::max(dmax, std::fabs(distances[i]));
-  for (int i = 0; i < nf; ++i) fmax = std::max(fmax, freqs[i]);
-  real = real && 2.0 * fmax / kC * nmax * dmax < 1e9;
-  std::vector<Region1DReal> rr(nd);
-  std::vector<double> x2(nf);
-  if (real) {
-    for (int j = 1; j < nd; ++j) {
-      const double nl = std::sqrt(e[j].real());
-      rr[j] = {nl, 1.0 / nl, (1.0 / e[j - 1].real() - 1.0 / e[j].real()) / 2.0};
-    }
-    for (int i = 0; i < nf; ++i) x2[i] = 2.0 * freqs[i] / kC;   // 2 / lambda: k0 = pi x2 n
-  }
-  TCKS(d_rg.alloc(h, real ? sizeof(Region1DReal) * nd : sizeof(Region1D) * nd));
-  if (real)
-    TCK(cudaMemcpyAsync(d_rg.p, rr.data(), sizeof(Region1DReal) * nd, cudaMemcpyHostToDevice, st));
-  else
-    TCK(cudaMemcpyAsync(d_rg.p, rg.data(), sizeof(Region1D) * nd, cudaMemcpyHostToDevice, st));
+  TCKS(d_rg.alloc(h, sizeof(Region1D) * nd));
+  TCK(cudaMemcpyAsync(d_rg.p, rg.data(), sizeof(Region1D) * nd, cudaMemcpyHostToDevice, st));
   TCKS(d_f.alloc(h, sizeof(double) * nf));
-  TCK(cudaMemcpyAsync(d_f.p, real ? x2.data() : freqs, sizeof(double) * nf, cudaMemcpyHostToDevice, st));
+  TCK(cudaMemcpyAsync(d_f.p, freqs, sizeof(double) * nf, cudaMemcpyHostToDevice, st));
   if (out_boost) TCKS(d_b.alloc(h, sizeof(double2) * npts));
   TCKS(d_b2.alloc(h, sizeof(double) * npts));
   bf::note_launch();
   tf_mark(h, 0);
-  const unsigned nblk = (unsigned)((npts + 255) / 256);
-  double2* db = out_boost ? d_b.as<double2>() : nullptr;
-  if (real)
-    k_tf1d_real<<<nblk, 256, 0, st>>>(d_dist.as<double>(), nd, d_rg.as<Region1DReal>(), 1.0 / std::sqrt(e[0].real()),
-                                      d_f.as<double>(), nf, nconf,
-                                      emit ? make_double2(emit[0], emit[1]) : make_double2(1.0, 0.0), db,
-                                      d_b2.as<double>());
-  else
-    k_tf1d<<<nblk, 256, 0, st>>>(d_dist.as<double>(), nd, d_rg.as<Region1D>(), d_f.as<double>(), nf, nconf, db,
-                                 d_b2.as<double>());
+  k_tf1d<<<(unsigned)((npts + 255) / 256), 256, 0, st>>>(d_dist.as<double>(), nd, d_rg.as<Region1D>(),
+                                                          d_f.as<double>(), nf, nconf,
+                                                          out_boost ? d_b.as<double2>() : nullptr, d_b2.as<double>());
   TCK(cudaGetLastError());
   tf_mark(h, 1);
   if (h->profiling) {
