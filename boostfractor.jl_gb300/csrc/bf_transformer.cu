@@ -1550,12 +1550,14 @@ __global__ void __launch_bounds__(1024) k_chain_df(const float2* P, const float2
 //   * k_invert_reg inverts T22 in complex64: the correction's approximate inverse;
 //   * k_refine evaluates residuals in double-float (the arithmetic of
 //     k_chain_df, on vectors) and corrects x until the next correction would be
-//     below 1e-9 |x|, 3 to 4 residuals;
+//     below 1e-13 |x|, or is the residual's own rounding: no less than T in
+//     double-float and an FP64 LU give, 3 to 5 residuals (at 1e-9, one less,
+//     x was off by up to 3e-10 where they are at 1e-13);
 //   * frequencies that do not converge (an ill-conditioned T22, a NaN) are
 //     marked and solved as before (k_chain_df and the FP64 LU).
 // 64 modes, 41 regions, 1024 frequencies: chain and boundary solve 38.5 + 3.3 ms
-// with T in double-float; 6.5 ms here (chain 4.1, 85 GFMA at 0.55 of the FP32
-// rate, inverse 0.2, residuals 2.2).
+// with T in double-float; 7.4 ms here (chain 4.1, 85 GFMA at 0.55 of the FP32
+// rate, inverse 0.2, residuals 3.0).
 template <int NB>
 __global__ void __launch_bounds__((NB / 2) * (NB / 4), NB == 64 ? 1 : 4)
     k_chain_f32(const float2* P, const float2* Pinv, const ChainRegionDF* cr, int nd, int nm, float2* T22out) {
@@ -1662,7 +1664,7 @@ __global__ void __launch_bounds__((NB / 2) * (NB / 4), NB == 64 ? 1 : 4)
 // axion beam's boost, 1 the reflection.  8 lanes a matrix row, 4 rows a warp,
 // P's rows then inverse(P)'s; a region's entries are loaded while the region
 // before is finished.  failed[f] is set when the iteration does not converge.
-constexpr int kRefineThreads = 512, kRefineMax = 8;
+constexpr int kRefineThreads = 512, kRefineMax = 12;
 __global__ void __launch_bounds__(kRefineThreads, 2)
     k_refine(const float2* P, const float2* Pinv, const float2* X, const ChainRegionDF* cr, int nd, int nm,
              const double2* emit, const double2* reflect, double2* boost, double2* refl, double* beta2, int* failed) {
@@ -1694,7 +1696,7 @@ __global__ void __launch_bounds__(kRefineThreads, 2)
         m[t][i] = out[t] >= 0 && l8 + 8 * i < nm ? row[t][(size_t)j * n2 + l8 + 8 * i] : make_float2(0.f, 0.f);
   };
   float last = 0.f;
-  bool ok = false;
+  bool ok = false, fell = false;
   for (int it = 0; it < kRefineMax && !ok; ++it) {
     // the residual: the vector (reflect or 0, x) through the regions, nd - 1 to 1
     fetch(nd - 1);
@@ -1768,9 +1770,12 @@ __global__ void __launch_bounds__(kRefineThreads, 2)
     }
     __syncthreads();
     const float dn = red[0][0], xn = red[0][1];
-    // the next correction is about dn (dn / last); the first one (x itself) has no rate
-    if (dn == 0.f || (it > 0 && dn < 0.1f * last && dn * (dn / last) <= 1e-9f * xn)) ok = true;
+    // the next correction is about dn (dn / last); the first one (x itself) has no rate; one that is small and stopped
+    // falling is the residual's rounding
+    const bool falls = it > 0 && dn < 0.1f * last;
+    if (dn == 0.f || (falls ? dn * (dn / last) <= 1e-13f * xn : fell && dn <= 1e-6f * xn)) ok = true;
     else if (!(dn < INFINITY) || (it > 0 && !(dn < 0.5f * last))) break;   // not contracting
+    fell = falls;
     last = dn;
     __syncthreads();
   }
