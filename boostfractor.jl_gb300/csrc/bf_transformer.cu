@@ -1546,8 +1546,11 @@ __global__ void __launch_bounds__(1024) k_chain_df(const float2* P, const float2
 // vector (reflect or 0, x) plus the axion terms is T21 u + T22 x + axion_beam,
 // two matrix-vector products a region.  So
 //   * k_chain_f32 forms T in complex64 (its error, amplified by cond(T22),
-//     is ~1e-3 of x);
-//   * k_invert_reg inverts T22 in complex64: the correction's approximate inverse;
+//     is ~1e-3 of x) and scales T22's rows and columns by powers of two to a
+//     largest entry near 1: evanescent modes' grow by e^(kappa dz) a region (20
+//     disks of eps 24, 24 radial modes: 5e25), and a pivot above 1.8e19 has no
+//     square, hence no reciprocal, in FP32;
+//   * k_invert_reg inverts it in complex64: the correction's approximate inverse;
 //   * k_refine evaluates residuals in double-float (the arithmetic of
 //     k_chain_df, on vectors) and corrects x until the next correction would be
 //     below 1e-13 |x|, or is the residual's own rounding: no less than T in
@@ -1560,7 +1563,8 @@ __global__ void __launch_bounds__(1024) k_chain_df(const float2* P, const float2
 // rate, inverse 0.2, residuals 3.0).
 template <int NB>
 __global__ void __launch_bounds__((NB / 2) * (NB / 4), NB == 64 ? 1 : 4)
-    k_chain_f32(const float2* P, const float2* Pinv, const ChainRegionDF* cr, int nd, int nm, float2* T22out) {
+    k_chain_f32(const float2* P, const float2* Pinv, const ChainRegionDF* cr, int nd, int nm, float2* T22out,
+                int* scales) {
   constexpr int NT = (NB / 2) * (NB / 4), CG = NB / 4, UP = NB + 2;
   extern __shared__ __align__(16) unsigned char sm[];
   float2* M = reinterpret_cast<float2*>(sm);            // [2][P, inverse(P)][NB][NB]
@@ -1653,11 +1657,42 @@ __global__ void __launch_bounds__((NB / 2) * (NB / 4), NB == 64 ? 1 : 4)
     }
     __syncthreads();
   }
+  // row r by 2^-er, then column c by 2^-ec: scales[f][0 .. nm) = er, [nm .. 2 nm) = ec; magnitudes
+  // compared as bits, where a NaN is the largest (and, like an infinity or a zero, is not scaled)
+  auto size = [](float2 z) { return max(__float_as_int(fabsf(z.x)), __float_as_int(fabsf(z.y))); };
+  auto expo = [](int m) { return m == 0 || m >= 0x7f800000 ? 0 : ilogbf(__int_as_float(m)); };
+  auto scale = [](float2& z, int e) { z = make_float2(ldexpf(z.x, -e), ldexpf(z.y, -e)); };
+  int* cmax = reinterpret_cast<int*>(Us);
+  int* sc = scales + (size_t)f * 2 * nm;
+  for (int c = tid; c < NB; c += NT) cmax[c] = 0;
+  __syncthreads();
 #pragma unroll
-  for (int r = 0; r < 2; ++r)
+  for (int r = 0; r < 2; ++r) {
+    int m = 0;
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
-      if (r0 + r < nm && col(i) < nm) T22out[(size_t)f * n2 + (r0 + r) * nm + col(i)] = t2[r][i];
+    for (int i = 0; i < 4; ++i) m = max(m, size(t2[r][i]));
+#pragma unroll
+    for (int o = 1; o < CG; o <<= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, o, CG));
+    const int e = expo(m);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      scale(t2[r][i], e);
+      if (r0 + r < nm) atomicMax(cmax + col(i), size(t2[r][i]));
+    }
+    if (tid % CG == 0 && r0 + r < nm) sc[r0 + r] = e;
+  }
+  __syncthreads();
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const int e = expo(cmax[col(i)]);
+    if (r0 == 0 && col(i) < nm) sc[nm + col(i)] = e;
+#pragma unroll
+    for (int r = 0; r < 2; ++r)
+      if (r0 + r < nm && col(i) < nm) {
+        scale(t2[r][i], e);
+        T22out[(size_t)f * n2 + (r0 + r) * nm + col(i)] = t2[r][i];
+      }
+  }
 }
 
 // Refinement of one (frequency, right-hand side) per CTA: blockIdx.y = 0 the
@@ -1666,11 +1701,12 @@ __global__ void __launch_bounds__((NB / 2) * (NB / 4), NB == 64 ? 1 : 4)
 // before is finished.  failed[f] is set when the iteration does not converge.
 constexpr int kRefineThreads = 512, kRefineMax = 12;
 __global__ void __launch_bounds__(kRefineThreads, 2)
-    k_refine(const float2* P, const float2* Pinv, const float2* X, const ChainRegionDF* cr, int nd, int nm,
-             const double2* emit, const double2* reflect, double2* boost, double2* refl, double* beta2, int* failed) {
+    k_refine(const float2* P, const float2* Pinv, const float2* X, const int* scales, const ChainRegionDF* cr, int nd,
+             int nm, const double2* emit, const double2* reflect, double2* boost, double2* refl, double* beta2, int* failed) {
   constexpr int NW = kRefineThreads / 32, TASKS = 2 * 64 / 4 / NW;   // rows of 64 modes: 2 tasks of 4 a warp
   __shared__ DFc vt[64], vb[64], pq[128], x[64], em[64];
-  __shared__ float red[2][2];
+  __shared__ float2 rs[64];   // the residual, its rows scaled like T22's
+  __shared__ float red[4];    // largest |d|, |x|, scaled |d|, scaled residual
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, l8 = lane & 7, f = blockIdx.x;
   const bool back = blockIdx.y == 1;
   const int n2 = nm * nm;
@@ -1745,15 +1781,25 @@ __global__ void __launch_bounds__(kRefineThreads, 2)
       __syncthreads();
     }
     // d = X r, x -= d
-    if (tid < 4) red[tid >> 1][tid & 1] = 0.f;
+    if (tid < 4) red[tid] = 0.f;
+    __syncthreads();
+    // non-negative floats order like their bits; a NaN orders above all
+    auto largest = [&](int i, float re, float im) {
+      atomicMax(reinterpret_cast<int*>(red + i), __float_as_int(fabsf(re) + fabsf(im)));
+    };
+    if (tid < nm) {
+      const int e = scales[(size_t)f * 2 * nm + tid];
+      rs[tid] = make_float2(ldexpf(vb[tid].rh, -e), ldexpf(vb[tid].ih, -e));
+      largest(3, rs[tid].x, rs[tid].y);
+    }
     __syncthreads();
     for (int r = 4 * warp + (lane >> 3); r < (nm + 3) / 4 * 4; r += 4 * NW) {
       float2 d = make_float2(0.f, 0.f);
       if (r < nm)
         for (int k = l8; k < nm; k += 8) {
           const float2 a = X[(size_t)f * n2 + r * nm + k];
-          d.x = fmaf(a.x, vb[k].rh, fmaf(-a.y, vb[k].ih, d.x));
-          d.y = fmaf(a.x, vb[k].ih, fmaf(a.y, vb[k].rh, d.y));
+          d.x = fmaf(a.x, rs[k].x, fmaf(-a.y, rs[k].y, d.x));
+          d.y = fmaf(a.x, rs[k].y, fmaf(a.y, rs[k].x, d.y));
         }
 #pragma unroll
       for (int o = 1; o < 8; o <<= 1) {
@@ -1761,19 +1807,24 @@ __global__ void __launch_bounds__(kRefineThreads, 2)
         d.y += __shfl_xor_sync(0xffffffffu, d.y, o);
       }
       if (l8 == 0 && r < nm) {
+        largest(2, d.x, d.y);
+        const int e = scales[(size_t)f * 2 * nm + nm + r];
+        d = make_float2(ldexpf(d.x, -e), ldexpf(d.y, -e));
         const DFc n = dfc_add(x[r], DFc{-d.x, 0.f, -d.y, 0.f});
         x[r] = n;
-        // non-negative floats order like their bits; a NaN orders above all
-        atomicMax(reinterpret_cast<int*>(&red[0][0]), __float_as_int(fabsf(d.x) + fabsf(d.y)));
-        atomicMax(reinterpret_cast<int*>(&red[0][1]), __float_as_int(fabsf(n.rh) + fabsf(n.ih)));
+        largest(0, d.x, d.y);
+        largest(1, n.rh, n.ih);
       }
     }
     __syncthreads();
-    const float dn = red[0][0], xn = red[0][1];
+    const float dn = red[0], xn = red[1];
+    // The scaled T22's entries are below 2, so a residual is at most 4 nm times the correction that removes it: one
+    // above twice that has parts that X does not see.
+    const bool seen = red[3] <= 8.f * nm * red[2];
     // the next correction is about dn (dn / last); the first one (x itself) has no rate; one that is small and stopped
     // falling is the residual's rounding
     const bool falls = it > 0 && dn < 0.1f * last;
-    if (dn == 0.f || (falls ? dn * (dn / last) <= 1e-13f * xn : fell && dn <= 1e-6f * xn)) ok = true;
+    if (seen && (dn == 0.f || (falls ? dn * (dn / last) <= 1e-13f * xn : fell && dn <= 1e-6f * xn))) ok = true;
     else if (!(dn < INFINITY) || (it > 0 && !(dn < 0.5f * last))) break;   // not contracting
     fell = falls;
     last = dn;
@@ -3320,7 +3371,7 @@ static int tf_run_t(bf_handle* h, bf_stack* s, bf_modes* md, int nf, const doubl
   TCKS(T22.alloc(h, sizeof(double2) * (size_t)nf * nm * nm));
   TCKS(ax.alloc(h, sizeof(double2) * (size_t)nf * nm));
   // the chain's factors as double-floats
-  DBuf d_crd, d_failed, T21df, T22df;
+  DBuf d_crd, d_failed, d_scales, T21df, T22df;
   int* failed = nullptr;   // refinement: the frequencies it leaves to the chain in double-float
   auto split_regions = [&](DBuf& d) -> int {
     static_assert(sizeof(ChainRegionDF) % sizeof(float4) == 0, "copied by 16 bytes");
@@ -3407,6 +3458,7 @@ static int tf_run_t(bf_handle* h, bf_stack* s, bf_modes* md, int nf, const doubl
       TCKS(T21df.ensure(h, n22));
       TCKS(T22df.ensure(h, n22));
       TCKS(d_failed.alloc(h, sizeof(int) * (nf + 1)));   // and a singularity word nobody reads
+      TCKS(d_scales.alloc(h, sizeof(int) * 2 * (size_t)nf * nm));
       TCK(cudaMemsetAsync(d_failed.p, 0, sizeof(int) * (nf + 1), st));
       failed = d_failed.as<int>();
       TCKS(split_regions(d_crd));
@@ -3416,7 +3468,7 @@ static int tf_run_t(bf_handle* h, bf_stack* s, bf_modes* md, int nf, const doubl
         TCK(cudaFuncSetAttribute(k_chain_f32<NB>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxDynSmem));
         bf::note_launch();
         k_chain_f32<NB><<<nf, (NB / 2) * (NB / 4), sm32, st>>>(Pd, Pinv.as<D2>(), d_crd.as<ChainRegionDF>(), nd, nm,
-                                                              T21df.as<float2>());
+                                                              T21df.as<float2>(), d_scales.as<int>());
         TCK(cudaGetLastError());
         bf::note_launch();
         k_invert_reg<NB><<<dim3(1, nf), (NB / 4) * (NB / 4), 0, st>>>(T21df.as<float2>(), T22df.as<float2>(), 1, 0, nm,
@@ -3427,9 +3479,9 @@ static int tf_run_t(bf_handle* h, bf_stack* s, bf_modes* md, int nf, const doubl
       TCKS(nm <= 32 ? run(std::integral_constant<int, 32>()) : run(std::integral_constant<int, 64>()));
       bf::note_launch();
       k_refine<<<dim3(nf, reflect ? 2 : 1), kRefineThreads, 0, st>>>(
-          Pd, Pinv.as<D2>(), T22df.as<float2>(), d_crd.as<ChainRegionDF>(), nd, nm, d_em.as<double2>(),
-          reflect ? d_refl.as<double2>() : nullptr, boost.as<double2>(), reflect ? refl.as<double2>() : nullptr,
-          b2.as<double>(), failed);
+          Pd, Pinv.as<D2>(), T22df.as<float2>(), d_scales.as<int>(), d_crd.as<ChainRegionDF>(), nd, nm,
+          d_em.as<double2>(), reflect ? d_refl.as<double2>() : nullptr, boost.as<double2>(),
+          reflect ? refl.as<double2>() : nullptr, b2.as<double>(), failed);
       TCK(cudaGetLastError());
     }
     TCK(cudaFuncSetAttribute(k_chain_df, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxDynSmem));
