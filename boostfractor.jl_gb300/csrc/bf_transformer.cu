@@ -2314,16 +2314,21 @@ static int tf_setup(bf_handle* h, bf_stack* s, bf_modes* md, int mode, TfCache**
       std::vector<double> sum(2 * c.T);
       TCK(cudaMemcpyAsync(sum.data(), d_sum.p, sizeof(double) * sum.size(), cudaMemcpyDeviceToHost, st));
       TCK(cudaStreamSynchronize(st));
-      // A row's product with the phasors (at most 1) is at most its sum of sizes.  Zero is what four units in the
-      // last place of the largest row could not show: rows that cancel by symmetry sum to 0.2 to 1 of them, the
-      // least of the others to 1e14.
-      const double zero = 4 * DBL_EPSILON * *std::max_element(sum.begin(), sum.end());
+      // A row's product with the phasors is at most its sum of sizes times the largest of them.  The rounding of row
+      // (m, m') scales with both modes' transforms, whose sizes the diagonals' real rows give (patterns come in any
+      // scale): zero is what four units in the last place of their geometric mean could not show.  Rows that cancel by
+      // symmetry sum to 0.2 to 1 of them, the least of the others to 1e14; phasors above 1 (negative distances, gain)
+      // would multiply the rounding that is left out, too.
+      std::vector<double> diag(nm);
+      for (int t = 0, m = 0; m < nm; t += nm - m++) diag[m] = sum[2 * t];
       std::vector<int> rows, map(2 * c.T, -1);
-      for (int r = 0; r < 2 * c.T; ++r)
-        if (!(sum[r] <= zero) || rows.empty()) {
-          map[r] = (int)rows.size();
-          rows.push_back(r);
-        }
+      for (int t = 0, m = 0; m < nm; ++m)
+        for (int mp = m; mp < nm; ++mp, ++t)
+          for (int r = 2 * t; r < 2 * t + 2; ++r)
+            if (!(sum[r] <= 4 * DBL_EPSILON * std::sqrt(diag[m]) * std::sqrt(diag[mp])) || (m == mp && r == 2 * t)) {
+              map[r] = (int)rows.size();
+              rows.push_back(r);
+            }
       c.Rw = (int)rows.size();
       c.Mw = (c.Rw + 127) / 128 * 128;
       TCKS(c.rowmap.alloc(h, sizeof(int) * map.size()));
