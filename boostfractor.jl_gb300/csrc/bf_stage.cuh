@@ -558,7 +558,7 @@ __device__ __forceinline__ void joint_mix(const FusedArgs<C>& a, const StepDesc&
 #pragma unroll
     for (int k = 0; k < K; ++k) {
       const int i = b + k * is;
-      if (i >= plane) continue;
+      if (i >= end) continue;
       if (tmA) tA[k] = tmA[i];
       if (tmB) tB[k] = tmB[i];
       if (!pa) A[k] = stA ? stA[i] : czero<C>();
@@ -572,7 +572,7 @@ __device__ __forceinline__ void joint_mix(const FusedArgs<C>& a, const StepDesc&
 #pragma unroll
     for (int k = 0; k < K; ++k) {
       const int i = b + k * is;
-      if (i >= plane) continue;
+      if (i >= end) continue;
       if (tmA) A[k] = cmul(A[k], tA[k]);
       if (tmB) B[k] = cmul(B[k], tB[k]);
       if (stA) {
