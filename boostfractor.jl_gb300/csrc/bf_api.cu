@@ -1043,6 +1043,11 @@ extern "C" int bf_autotune_report(char* out, int cap) {
 
 extern "C" int bf_test_force_fused_variant(int v) { return g_force_variant.exchange(v); }
 
+// Test hook: while non-zero, the barriers of a run of split stages wait for one arrival more than there are CTAs, for
+// ~0.1 s instead of ~2 s, and the solve returns BF_ERR_TIMEOUT.
+static std::atomic<int> g_run_late{0};
+extern "C" int bf_test_run_withhold_arrival(int on) { return g_run_late.exchange(on ? 1 : 0); }
+
 template <typename C>
 static int fused_autotune(bf_handle* h, const Workspace& w, const bf::FusedArgs<C>& a, int grid, int N, bool fp64,
                           cudaStream_t st, int* out) {
@@ -1327,6 +1332,10 @@ static int run_fused(bf_handle* h, bf_stack* s, const std::string& key,
   }
   prof_mark(h, 1);
   const unsigned long long l1 = bf::launch_count();
+  if (g_run_late.load()) {
+    a.run_late = 1;
+    a.run_limit = 200000000LL;
+  }
   auto run_stages = [&]() -> int {
     auto in_run = [&](size_t k) {
       return fp64 && a.mg && w.stage_len[k] > 0 && bf::split_stage((int)w.stage_len[k], nf) &&
@@ -1362,7 +1371,7 @@ static int run_fused(bf_handle* h, bf_stack* s, const std::string& key,
     const void* ptrs[] = {a.state, a.phasor, a.tilt, a.tilt_idx, a.mask, a.coefs, a.exitacc, a.addbuf,
                           a.err, w.steps.p, a.mg, a.tab_idx, w.run.p};
     const long long ints[] = {h->sm_cap, nf, a.nbx, a.nby, a.nslots, a.ntab, a.fold, a.ntilt, N, (long long)fp64,
-                              (long long)w.stage_off.size(), h->device, a.variant};
+                              (long long)w.stage_off.size(), h->device, a.variant, (long long)a.run_late};
     gkey.append(reinterpret_cast<const char*>(ptrs), sizeof(ptrs));
     gkey.append(reinterpret_cast<const char*>(ints), sizeof(ints));
     gkey.append(reinterpret_cast<const char*>(w.stage_off.data()), sizeof(size_t) * w.stage_off.size());
@@ -1809,7 +1818,7 @@ static int check_device_error(bf_handle* h) {
   int err = 0;
   CK(cudaMemcpyAsync(&err, h->d_scalar + 1, sizeof(int), cudaMemcpyDeviceToHost, h->stream()));
   CK(cudaStreamSynchronize(h->stream()));
-  if (err) return fail(h, BF_ERR_TIMEOUT, "a bounded wait for a shared-memory copy expired in the bounce kernel");
+  if (err) return fail(h, BF_ERR_TIMEOUT, "a bounded wait of the bounce stages' grid barrier expired");
   return BF_OK;
 }
 

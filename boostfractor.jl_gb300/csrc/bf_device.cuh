@@ -55,6 +55,8 @@ struct FusedArgs {
   unsigned* run_bar = nullptr;
   int run_len = 0;
   int max_ctas = 0;               // 0 = no limit on the run's CTAs
+  long long run_limit = 4000000000LL;   // cycles that a barrier waits: ~2 s
+  unsigned run_late = 0;          // a test's arrivals that never come
 };
 
 // Variants of the fused stage kernel for stages that do not take the

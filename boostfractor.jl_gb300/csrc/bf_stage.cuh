@@ -712,8 +712,8 @@ __global__ void __launch_bounds__(kSplitThreads) k_split_phase(FusedArgs<cplx_t<
 // launches, 29 us here, of which the barriers are 4 (1.3 us each).
 
 // Every CTA of the (cooperatively launched) grid arrives; false when the wait
-// gave up after ~2 s or another CTA's did.
-__device__ __forceinline__ bool run_barrier(unsigned* bar, unsigned target, int* err) {
+// gave up after `limit` cycles or another CTA's did.
+__device__ __forceinline__ bool run_barrier(unsigned* bar, unsigned target, long long limit, int* err) {
   __syncwarp();
   bool ok = true;
   if ((threadIdx.x & 31) == 0) {
@@ -728,7 +728,7 @@ __device__ __forceinline__ bool run_barrier(unsigned* bar, unsigned target, int*
         ok = false;
         break;
       }
-      if (clock64() - t0 > 4000000000LL) {
+      if (clock64() - t0 > limit) {
         atomicExch(err, 1);
         atomicExch(bar + 1, 1u);
         ok = false;
@@ -796,7 +796,7 @@ __global__ void __launch_bounds__(32) k_split_run(FusedArgs<cplx_t<R>> a) {
       }
       if (k + 1 == a.run_len && ph == 2) break;
       target += gridDim.x;
-      if (!run_barrier(a.run_bar, target, a.err)) return;
+      if (!run_barrier(a.run_bar, target + a.run_late, a.run_limit, a.err)) return;
     }
   }
 }

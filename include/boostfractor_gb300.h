@@ -484,6 +484,11 @@ int bf_test_force_fused_variant(int variant);
  * bounded wait runs out after ~2 s and the solve returns BF_ERR_TIMEOUT with
  * the CUDA context intact: the test of the kernel's bounded waits. */
 int bf_test_tc_withhold_loads(int on);
+/* No counterpart in the reference.  While `on` is non-zero, the grid barriers
+ * of FP64 bounce stages that run in one launch (few frequencies) wait for one
+ * arrival that never comes; they give up after ~0.1 s (~2 s otherwise) and the
+ * solve returns BF_ERR_TIMEOUT.  Returns the previous setting. */
+int bf_test_run_withhold_arrival(int on);
 
 #ifdef __cplusplus
 }
