@@ -357,9 +357,13 @@ __device__ __forceinline__ void split_tf32(float x, float& hi, float& lo) {
 // exp(i im) - 1 and exp(re) - 1 without branches (sincosf's and expm1f's keep a
 // thread's entries from overlapping), for |im| up to 80: im less a whole number
 // q of half turns in two steps, then sin and cos of half the rest r, |r / 2| at
-// most a quarter of pi, by the single-precision series of Cephes (Moshier):
-// cos im - 1 = -2 sin^2 or -2 cos^2 of r / 2 and sin im = +-2 sin cos for q even or
-// odd keep it accurate relative to its own size.
+// most a quarter of pi, by the single-precision series of Cephes (Moshier), as
+// -2 sin^2 or -2 cos^2 of r / 2 and +-2 sin cos for q even or odd.  Accurate to
+// 1e-7 of themselves but near whole turns (not near 0), where what the two
+// steps leave of pi counts: off by up to 1e-9 there.  The entries are sums of
+// terms of the order of 1, and their error is that of the phases in float32:
+// 9.96e-9 rms against 64 bits at 8 mm (8 modes, 128^2; with sincosf and expm1f
+// 1.00e-8), 4.9e-8 at 6 cm (5.0e-8).
 __device__ __forceinline__ float2 phase_m1(float im) {
   const float kMagic = 12582912.0f;   // 1.5 2^23: adding it rounds to a whole number
   const float m = fmaf(im, 0.318309886f, kMagic), q = m - kMagic;
@@ -375,7 +379,8 @@ __device__ __forceinline__ float2 phase_m1(float im) {
   const float a = odd ? c : s, b = odd ? -s : c;
   return make_float2(-2.0f * a * a, 2.0f * a * b);
 }
-// exp(x) - 1 for x <= 80: x less a whole number of ln 2, the Taylor series of the rest
+// exp(x) - 1 for x <= 80: x less a whole number of ln 2 (in Cephes' two parts), the Taylor series of the rest; 1.1e-7 of
+// itself at most
 __device__ __forceinline__ float expm1_series(float x) {
   const float kMagic = 12582912.0f;
   x = fmaxf(x, -80.0f);
