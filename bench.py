@@ -237,6 +237,22 @@ def measured_tf32_peak():
     return 1900.0 / 2.0, "half of fallback bf16"
 
 
+def fp32_peak():
+    """FP32 FFMA rate in TFLOP/s."""
+    sp = simt_peaks()
+    if sp and sp.get("fp32_ffma_tflops"):
+        return float(sp["fp32_ffma_tflops"]), "measured (FFMA probe, profiles/simt_peaks.json)"
+    return 78.0, "nominal"
+
+
+def stage_transform(w):
+    """(pixels of the box that the disk mask reaches, length of the transforms that the bounce stages run on it): a
+    propagation's input and needed output lie in the box, so the shortest length >= 2 box - 1 gives its field."""
+    mask = w["X"][:, None] ** 2 + w["Y"][None, :] ** 2 < w["diskR"] ** 2
+    box = max(int(np.ptp(np.nonzero(mask.any(k))[0])) + 1 for k in (0, 1))
+    return box, min([m for m in (8, 16, 32, 40, 64, 80, 128, 160, 256) if m >= 2 * box - 1] + [len(w["X"])])
+
+
 def ncu_traffic():
     """DRAM bytes per propagation of the fused stage kernel from the committed ncu summary."""
     p = os.path.join(REPO, "profiles", "fused_stage_ncu.json")
@@ -348,19 +364,21 @@ def run_ours(args):
     ms_step = ms_total / args.steps
     value = replica_value(ms_total, args.steps, nf, ws)
 
-    # roofline of the fused stage kernel (bytes per propagation: read + write of
-    # the complex64 field, 2*N^2*8)
-    N = len(w["X"])
-    alg_bytes_per_prop = 2 * N * N * 8
-    achieved = alg_bytes_per_prop * props / (stage_ms / 1000.0) / 1e9
-    peak, peak_kind = measured_peaks()
+    # roofline of the fused stage kernel: 5 M log2 M flops a transform of the length M that runs, box rows forward and
+    # back and M columns forward and back a propagation, over the FP32 rate; the bytes that a propagation cannot do
+    # without (the box's complex64 field read and written) need a small part of the HBM rate
+    box, M = stage_transform(w)
+    fft_flops = props * (2 * M + 2 * box) * 5 * M * math.log2(M)
+    achieved = fft_flops / (stage_ms / 1000.0) / 1e12
+    hbm = 2 * box * box * 8 * props / (stage_ms / 1000.0) / 1e9
+    peak, peak_kind = fp32_peak()
     tr = ncu_traffic()
-    roof = {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
+    roof = {"bound": "fp32", "achieved": achieved, "peak": peak, "unit": "TFLOP/s",
             "frac": achieved / peak, "peak_source": peak_kind,
             "traffic": None if tr is None else tr * props / stage_launches,
-            "kernel": "k_fused_stage", "launch_avg_ms": stage_ms / max(stage_launches, 1),
-            "alg_bytes_per_launch": alg_bytes_per_prop * props / max(stage_launches, 1),
-            "fft_gflops": props * (2 * N + 2 * 38) * 5 * N * math.log2(N) / (stage_ms / 1000.0) / 1e9}
+            "kernel": "k_fused_stage", "transform": M, "box": box, "launch_avg_ms": stage_ms / max(stage_launches, 1),
+            "alg_bytes_per_launch": 2 * box * box * 8 * props / max(stage_launches, 1),
+            "hbm_gbs": hbm, "hbm_frac": hbm / measured_peaks()[0]}
 
     # ---- end to end through the one-shot C ABI call with host buffers
     import ctypes
@@ -1163,13 +1181,12 @@ def run_1d(args):
         errs.append(abs(b2[c, k] - ref) / ref)
     m1.close()
     h.close()
-    # FP64 roofline of k_tf1d: the explicit arithmetic of one region (complex
-    # products 6 flops, sums 2: axion term 10, boundary factors 28, propagation
-    # 12, phase argument 2 = 52 flops), not counting sincospi, over the FP64
-    # DFMA rate measured by `bench.py --workload peaks` (nominal 1.25 TFLOP/s
-    # without it)
+    # FP64 roofline of k_tf1d: the explicit arithmetic of one lossless region
+    # (axion term 6 flops, boundary factors 12, propagation 12, phase argument 2
+    # = 32), not counting sincospi, over the FP64 DFMA rate measured by
+    # `bench.py --workload peaks` (nominal 1.25 TFLOP/s without it)
     nregions = len(eps) - 1
-    flops = 52.0 * nregions * nconf * nf
+    flops = 32.0 * nregions * nconf * nf
     sp = simt_peaks()
     fp64_peak, fp64_src = ((float(sp["fp64_dfma_tflops"]), "measured (DFMA probe, profiles/simt_peaks.json)")
                            if sp and sp.get("fp64_dfma_tflops") else (1.25, "nominal"))
@@ -1185,7 +1202,7 @@ def run_1d(args):
             "roofline": {"bound": "fp64", "achieved": flops / (kms / 1000.0) / 1e12,
                          "peak": fp64_peak, "peak_source": fp64_src, "unit": "TFLOP/s",
                          "frac": flops / (kms / 1000.0) / 1e12 / fp64_peak,
-                         "kernel": "k_tf1d", "flops_per_region": 52, "note": "sincospi/exp not counted"},
+                         "kernel": "k_tf1d", "flops_per_region": 32, "note": "sincospi not counted"},
             "gpu_launches": args.steps, "clocks": clocks,
             "e2e": {"value": nconf * nf / wall, "unit": UNIT, "h2d_bytes_per_step": int(confs.nbytes + freqs.nbytes),
                     "d2h_bytes_per_step": int(b2.nbytes)}}

@@ -1559,8 +1559,8 @@ __global__ void __launch_bounds__(1024) k_chain_df(const float2* P, const float2
 //   * frequencies that do not converge (an ill-conditioned T22, a NaN) are
 //     marked and solved as before (k_chain_df and the FP64 LU).
 // 64 modes, 41 regions, 1024 frequencies: chain and boundary solve 38.5 + 3.3 ms
-// with T in double-float; 7.4 ms here (chain 4.1, 85 GFMA at 0.55 of the FP32
-// rate, inverse 0.2, residuals 3.0).
+// with T in double-float; 7.5 ms here (chain 4.1, FP32 pipe 60 % and shared
+// memory 77 % busy, inverse 0.2, residuals 3.2).
 template <int NB>
 __global__ void __launch_bounds__((NB / 2) * (NB / 4), NB == 64 ? 1 : 4)
     k_chain_f32(const float2* P, const float2* Pinv, const ChainRegionDF* cr, int nd, int nm, float2* T22out,
