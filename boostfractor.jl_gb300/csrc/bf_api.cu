@@ -1171,13 +1171,9 @@ static int run_fused(bf_handle* h, bf_stack* s, const std::string& key,
   // and comes out once at the exits
   const bool compact = N != n || (n & (n - 1)) != 0;
   const double alpha = compact ? M_PI * ((n % 2 == 0 ? 1.0 / n : 0.0) - 1.0 / N) : 0.0;
-  auto modulate = [&](std::vector<cd>& boxes) {
-    if (alpha == 0.0) return;
-    for (size_t i = 0; i < boxes.size(); ++i) {
-      const size_t p = i % plane;
-      const double t = alpha * (double)(p / s->nbx + p % s->nbx);
-      boxes[i] *= cd(std::cos(t), std::sin(t));
-    }
+  auto modulate = [&](DBuf& boxes, size_t total) -> int {
+    if (alpha != 0.0) CKL(bf::launch_modulate(boxes.as<double2>(), total, s->nbx, s->nby, alpha, st));
+    return BF_OK;
   };
   const int QW = fold ? N / 2 : N;
   const std::string full_key = key + "|v" + std::to_string(s->geo_version) + (fp64 ? "|d" : "|f");
@@ -1196,8 +1192,8 @@ static int run_fused(bf_handle* h, bf_stack* s, const std::string& key,
     w.exit_coef = p.exit_coef;
     w.tab_region = p.tab_region;
     if (compact) {
-      const std::vector<double> A = bf::compact_matrix(n, N, std::max(s->nbx, s->nby));
-      CKS(upload(h, w.compact_A, A.data(), sizeof(double) * A.size()));
+      CKS(w.compact_A.ensure(h, sizeof(double) * bf::compact_matrix_size(n, N)));
+      CKL(bf::launch_compact_matrix(w.compact_A.as<double>(), n, N, std::max(s->nbx, s->nby), st));
     }
     std::vector<int> tidx(w.ntab, -1), tregs;
     for (int t = 0; t < w.ntab; ++t) {
@@ -1212,15 +1208,15 @@ static int run_fused(bf_handle* h, bf_stack* s, const std::string& key,
     if (w.ntilt) CKS(upload(h, w.tregs, tregs.data(), sizeof(int) * w.ntilt));
     std::vector<cd> init((size_t)p.nslots * plane);
     for (int k = 0; k < p.nslots; ++k) std::copy(p.init[k].begin(), p.init[k].end(), init.begin() + k * plane);
-    modulate(init);
     CKS(upload_cd_as(h, w.init, init));
+    CKS(modulate(w.init, init.size()));
     w.nadd = (int)p.adds.size();
     if (w.nadd) {
       std::vector<cd> adds(p.adds.size() * plane);
       for (size_t k = 0; k < p.adds.size(); ++k) std::copy(p.adds[k].begin(), p.adds[k].end(), adds.begin() + k * plane);
-      modulate(adds);
       DBuf b_add64;
       CKS(upload_cd_as(h, b_add64, adds));
+      CKS(modulate(b_add64, adds.size()));
       CKS(w.add.alloc(h, csz * adds.size()));
       CKL(bf::launch_convert(b_add64.p, true, w.add.p, fp64, adds.size(), st));
       CK(cudaStreamSynchronize(st));

@@ -466,26 +466,29 @@ int compact_length(int box, bool fp64) {
 // A[q][a] (q over the non-negative wavenumbers of the n-point grid: q + 1/2 for
 // even n, q for odd n, in units of 2 pi / (n dx); a < M/2: the wavenumber
 // (a + 1/2) of the M-point transform): weight (2, or 1 at wavenumber 0) / (n M)
-// times sum_{|d| < box} cos(2 pi q' d / n) cos(2 pi a' d / M).
-std::vector<double> compact_matrix(int n, int M, int box) {
-  const int Q = (n + 1) / 2, H = M / 2;
+// times sum_{|d| < box} cos(2 pi q' d / n) cos(2 pi a' d / M).  On the device,
+// since a plan of a call of its own emission, or of a one-shot call, makes it
+// anew: on the host it took 0.15 ms at 128 and 1.2 ms at 256 points.
+__global__ void k_compact_matrix(double* A, int n, int M, int box) {
+  const int Q = (n + 1) / 2, H = M / 2, i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= Q * H) return;
+  const int q = i / H, a = i % H;
   const bool even = n % 2 == 0;
   // sum_{|d| < box} cos(theta d), theta / 2 = pi num / (2 n M)
   auto dirichlet = [&](long long num) {
     const double den = 2.0 * n * M;
-    const double s = sin(M_PI * (double)num / den);
     if (num % (2LL * n * M) == 0) return 2.0 * box - 1.0;
-    return sin(M_PI * (double)((num * (2LL * box - 1)) % (4LL * n * M)) / den) / s;
+    return sinpi((double)((num * (2LL * box - 1)) % (4LL * n * M)) / den) / sinpi((double)num / den);
   };
-  std::vector<double> A((size_t)Q * H);
-  for (int q = 0; q < Q; ++q)
-    for (int a = 0; a < H; ++a) {
-      // theta / 2 = pi (q'/n -+ a'/M), 2 q' and 2 a' whole
-      const long long x = (long long)(even ? 2 * q + 1 : 2 * q) * M, y = (long long)(2 * a + 1) * n;
-      const double sum = 0.5 * (dirichlet(x - y) + dirichlet(x + y));
-      A[(size_t)q * H + a] = (!even && q == 0 ? 1.0 : 2.0) / ((double)n * M) * sum;
-    }
-  return A;
+  // theta / 2 = pi (q'/n -+ a'/M), 2 q' and 2 a' whole
+  const long long x = (long long)(even ? 2 * q + 1 : 2 * q) * M, y = (long long)(2 * a + 1) * n;
+  A[i] = (!even && q == 0 ? 1.0 : 2.0) / ((double)n * M) * (0.5 * (dirichlet(x - y) + dirichlet(x + y)));
+}
+size_t compact_matrix_size(int n, int M) { return (size_t)((n + 1) / 2) * (M / 2); }
+int launch_compact_matrix(double* A, int n, int M, int box, cudaStream_t st) {
+  COUNT_LAUNCH();
+  k_compact_matrix<<<(unsigned)((compact_matrix_size(n, M) + 127) / 128), 128, 0, st>>>(A, n, M, box);
+  return (int)cudaGetLastError();
 }
 
 int launch_compact_table(bool fp64, void* out, int nfreq, const double* d_freqs, int ntab, int stride,
@@ -830,6 +833,21 @@ int launch_exit_combine(double2* out, const double2* full, const double2* direct
   size_t total = (size_t)nfreq * npix;
   COUNT_LAUNCH();
   k_exit_combine<<<grid1d(total), 256, 0, st>>>(out, full, direct, coef, nfreq, npix);
+  return (int)cudaGetLastError();
+}
+
+// boxes of nbx x nby pixels, `total` in all, times exp(i alpha (x + y)): what k_embed_box takes out again
+__global__ void k_modulate(double2* boxes, size_t total, int nbx, int plane, double alpha) {
+  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
+    const int p = (int)(i % plane);
+    boxes[i] = cmul(boxes[i], dcexp(0.0, alpha * (p / nbx + p % nbx)));
+  }
+}
+
+int launch_modulate(double2* boxes, size_t total, int nbx, int nby, double alpha, cudaStream_t st) {
+  if (!total) return 0;
+  COUNT_LAUNCH();
+  k_modulate<<<grid1d(total), 256, 0, st>>>(boxes, total, nbx, nbx * nby, alpha);
   return (int)cudaGetLastError();
 }
 

@@ -99,7 +99,8 @@ bool split_run_fits(int N, int nsteps, int nfreq);
 // within the box), 0 if there is none; the matrix that takes a grid's phasors
 // to that transform's spectrum.
 int compact_length(int box, bool fp64);
-std::vector<double> compact_matrix(int n, int M, int box);
+size_t compact_matrix_size(int n, int M);
+int launch_compact_matrix(double* A, int n, int M, int box, cudaStream_t st);
 
 // ---- split-TF32 tensor-core GEMM (bf_tcgemm.cu) --------------------------
 // out[z][n][m] (FP32) = sum over the z-th of `splits` K slices of
@@ -144,7 +145,7 @@ int launch_phasor_table(bool fp64, void* out, int nfreq, const double* d_freqs, 
                         const int* d_regions, const RegionGeo* d_geo, int N, const double* d_kX,
                         const double* d_kY, int fold, cudaStream_t st);
 // The same for a compact transform of length M on an n x n grid (always one
-// quadrant, M/2 x M/2); d_A = compact_matrix(n, M, box).
+// quadrant, M/2 x M/2); d_A: launch_compact_matrix(n, M, box).
 int launch_compact_table(bool fp64, void* out, int nfreq, const double* d_freqs, int ntab, int stride,
                          const int* d_regions, const RegionGeo* d_geo, int n, const double* d_kX, const double* d_kY,
                          const double* d_A, int M, cudaStream_t st);
@@ -180,6 +181,8 @@ int launch_convert(const void* in, bool in_fp64, void* out, bool out_fp64, size_
 // out[f][ny][nx] (complex128) = direct[ny][nx] + coef * full[f][ny][nx]
 int launch_exit_combine(double2* out, const double2* full, const double2* direct,
                         double2 coef, int nfreq, int npix, cudaStream_t st);
+// boxes[..][nby][nbx] *= exp(i alpha (x + y)), x and y from the box's corner
+int launch_modulate(double2* boxes, size_t total, int nbx, int nby, double alpha, cudaStream_t st);
 // embed box acc [f][nby][nbx] (FP64) times exp(-i alpha (x + y)), x and y from
 // the box's corner, into full grid [f][ny][nx] (FP64)
 int launch_embed_box(double2* full, const double2* box, int nfreq, int nx, int ny, int nbx,

@@ -108,7 +108,7 @@ struct StageGraph {
 // steady-state path) and the cached bounce plan.
 struct Workspace {
   DBuf freq, reg, phasor, tidx, tregs, tilt, init, state, add, coef, exitacc, steps, run, tmp, beta, mg;
-  DBuf tab_idx, compact_A;       // table of each region; compact_matrix
+  DBuf tab_idx, compact_A;       // table of each region; launch_compact_matrix
   DBuf exit_full[2], direct[2];
   std::string plan_key;  // solver/nmax/emission of the cached plan
   std::vector<size_t> stage_off, stage_len;
