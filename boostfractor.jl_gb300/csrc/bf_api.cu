@@ -1272,10 +1272,14 @@ static int run_fused(bf_handle* h, bf_stack* s, const std::string& key,
     CKS(w.tab_idx.ensure(h, sizeof(int) * w.ntab));
     CK(cudaMemcpyAsync(w.tab_idx.p, idx.data(), sizeof(int) * w.ntab, cudaMemcpyHostToDevice, st));
     CKS(w.phasor.ensure(h, csz * (size_t)nf * w.ntab * QW * QW));
-    if (compact)
+    if (compact) {
+      DBuf tmp;   // without it (a budget that it does not fit) a CTA a table
+      const size_t nb = bf::compact_tmp_bytes(n, N, (int)regs.size(), nf);
+      if (nb && nb <= (64u << 20) && tmp.alloc(h, nb) != BF_OK) h->err.clear();
       CKL(bf::launch_compact_table(fp64, w.phasor.p, nf, w.freq.as<double>(), (int)regs.size(), w.ntab,
-                                   w.reg.as<int>(), s->d_geo, n, s->dkX, s->dkY, w.compact_A.as<double>(), N, st));
-    else
+                                   w.reg.as<int>(), s->d_geo, n, s->dkX, s->dkY, w.compact_A.as<double>(), N,
+                                   tmp.as<double2>(), st));
+    } else
       CKL(bf::launch_phasor_table(fp64, w.phasor.p, nf, w.freq.as<double>(), (int)regs.size(), w.ntab,
                                   w.reg.as<int>(), s->d_geo, N, s->dkX, s->dkY, fold, st));
     if (w.ntilt) {

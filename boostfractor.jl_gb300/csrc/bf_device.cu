@@ -444,6 +444,52 @@ __global__ void __launch_bounds__(256) k_compact_table(C* out, const double* fre
   }
 }
 
+// The same in two launches for fewer tables than SMs (a call of one or few
+// frequencies): a CTA takes kSplitRows rows of D to T in global memory, then a
+// thread an entry of S, its sums in the order that k_compact_table has them.
+// One SM's FP64 pipe took 0.75 ms for a table of 256 points to length 160.
+constexpr int kSplitRows = 4;
+__global__ void __launch_bounds__(256) k_compact_rows(double2* T, const double* freqs, const int* regions,
+                                                      const RegionGeo* geo, int Q, int first, const double* kX,
+                                                      const double* kY, const double* A, int H) {
+  extern __shared__ __align__(16) unsigned char sm[];
+  double2* D = reinterpret_cast<double2*>(sm);   // [kSplitRows][Q]
+  const RegionGeo gg = geo[regions[blockIdx.x]];
+  const double2 k0 = k0_of(SPEED_OF_LIGHT / freqs[blockIdx.y], gg.eps_re, gg.eps_im);
+  const int x0 = blockIdx.z * kSplitRows, nx = min(kSplitRows, Q - x0);
+  for (int i = threadIdx.x; i < nx * Q; i += blockDim.x)
+    D[i] = phasor_value(k0, kX[first + x0 + i / Q], kY[first + i % Q], gg.dz);
+  __syncthreads();
+  double2* t0 = T + ((size_t)blockIdx.y * gridDim.x + blockIdx.x) * (size_t)(Q * H) + (size_t)x0 * H;
+  for (int i = threadIdx.x; i < nx * H; i += blockDim.x) {
+    const int r = i / H, b = i % H;
+    double2 t = make_double2(0.0, 0.0);
+    for (int q = 0; q < Q; ++q) {
+      const double w = A[q * H + b];
+      const double2 d = D[r * Q + q];
+      t.x = fma(d.x, w, t.x);
+      t.y = fma(d.y, w, t.y);
+    }
+    t0[i] = t;
+  }
+}
+template <typename C>
+__global__ void __launch_bounds__(128) k_compact_sums(C* out, const double2* T, int stride, const double* A, int Q, int H) {
+  const int e = blockIdx.z * blockDim.x + threadIdx.x;
+  if (e >= H * H) return;
+  const int a = e / H, b = e % H;
+  const double2* t0 = T + ((size_t)blockIdx.y * gridDim.x + blockIdx.x) * (size_t)(Q * H) + b;
+  double2 s = make_double2(0.0, 0.0);
+#pragma unroll 8
+  for (int r = 0; r < Q; ++r) {
+    const double w = A[r * H + a];
+    const double2 t = t0[(size_t)r * H];
+    s.x = fma(t.x, w, s.x);
+    s.y = fma(t.y, w, s.y);
+  }
+  out[((size_t)blockIdx.y * stride + blockIdx.x) * (size_t)(H * H) + a * H + folded_at(2 * H, b)] = from_d<C>(s);
+}
+
 // Smallest transform length of the kernels that is at least 2 box - 1.  Both the
 // input and the needed output of a propagation lie in the box, so only the
 // offsets |d| < box of the propagator's N x N convolution kernel are ever used:
@@ -491,12 +537,35 @@ int launch_compact_matrix(double* A, int n, int M, int box, cudaStream_t st) {
   return (int)cudaGetLastError();
 }
 
+// Columns of S that a CTA of k_compact_table takes.
+static int compact_slice(int H) { return H <= 40 ? H : H == 80 ? 40 : 32; }
+
+// Bytes of launch_compact_table's scratch, 0 where the tables fill the SMs and
+// are bound by the FP64 pipe either way.  Tables of 128 points to length 80, whole
+// solves of one bounce: 3 tables 371 us in two launches, 554 in one; 96 tables
+// 461 and 545.
+size_t compact_tmp_bytes(int n, int M, int ntab, int nfreq) {
+  const int Q = (n + 1) / 2, H = M / 2;
+  if ((long long)ntab * nfreq * (H / compact_slice(H)) >= sm_count()) return 0;
+  return sizeof(double2) * (size_t)ntab * nfreq * Q * H;
+}
+
 int launch_compact_table(bool fp64, void* out, int nfreq, const double* d_freqs, int ntab, int stride,
                          const int* d_regions, const RegionGeo* d_geo, int n, const double* d_kX, const double* d_kY,
-                         const double* d_A, int M, cudaStream_t st) {
+                         const double* d_A, int M, double2* tmp, cudaStream_t st) {
   if (ntab <= 0 || nfreq <= 0) return 0;
   const int Q = (n + 1) / 2, H = M / 2, first = n / 2;
-  const int BS = H <= 40 ? H : H == 80 ? 40 : 32;
+  if (tmp) {
+    COUNT_LAUNCH();
+    k_compact_rows<<<dim3(ntab, nfreq, (Q + kSplitRows - 1) / kSplitRows), 256, sizeof(double2) * kSplitRows * Q, st>>>(
+        tmp, d_freqs, d_regions, d_geo, Q, first, d_kX, d_kY, d_A, H);
+    COUNT_LAUNCH();
+    const dim3 grid(ntab, nfreq, (H * H + 127) / 128);
+    if (fp64) k_compact_sums<double2><<<grid, 128, 0, st>>>((double2*)out, tmp, stride, d_A, Q, H);
+    else k_compact_sums<float2><<<grid, 128, 0, st>>>((float2*)out, tmp, stride, d_A, Q, H);
+    return (int)cudaGetLastError();
+  }
+  const int BS = compact_slice(H);
   const size_t smem = sizeof(double2) * kChunk * (Q + BS);
   dim3 grid(ntab, nfreq, H / BS);
   auto go = [&](auto* o, auto e) {

@@ -145,10 +145,11 @@ int launch_phasor_table(bool fp64, void* out, int nfreq, const double* d_freqs, 
                         const int* d_regions, const RegionGeo* d_geo, int N, const double* d_kX,
                         const double* d_kY, int fold, cudaStream_t st);
 // The same for a compact transform of length M on an n x n grid (always one
-// quadrant, M/2 x M/2); d_A: launch_compact_matrix(n, M, box).
+// quadrant, M/2 x M/2); tmp: compact_tmp_bytes of scratch, or null; d_A: launch_compact_matrix(n, M, box).
+size_t compact_tmp_bytes(int n, int M, int ntab, int nfreq);
 int launch_compact_table(bool fp64, void* out, int nfreq, const double* d_freqs, int ntab, int stride,
                          const int* d_regions, const RegionGeo* d_geo, int n, const double* d_kX, const double* d_kY,
-                         const double* d_A, int M, cudaStream_t st);
+                         const double* d_A, int M, double2* tmp, cudaStream_t st);
 // tilt[f][m][nby][nbx] = exp(-i k0 (tx x + ty y)) * exp(-i k0 surf) for map m of region regions[m]
 int launch_tilt_table(bool fp64, void* out, int nfreq, const double* d_freqs, int nmaps,
                       const int* d_regions, const RegionGeo* d_geo, int nbx, int nby, int bx0,
