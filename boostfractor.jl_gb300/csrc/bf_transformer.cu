@@ -2174,6 +2174,7 @@ struct TfCache {
   int Rw = 0, Mw = 0;
   int T = 0;
   bool herm_w = false;
+  bool dependent = false;   // the modes depend on one another beyond rounding
   // tensor-core path: the real rows of both classes as TF32 hi/lo pairs [Mp][Kp],
   // [Mp][Kdp] (rows padded to a multiple of 128, K to a multiple of 32) and
   // their FP64 row sums (gW, gV)
@@ -2197,6 +2198,32 @@ static size_t tf_cache_bytes(const void* p) {
 
 static thread_local double g_tf_gemm_flops = 0.0;   // executed real flops of the class GEMMs of this thread's last solve
 static int launch_rgemm(bf_handle* h, const float* A, const float2* B, double2* Hm, int R, int K, int N);
+
+// Whether nm vectors are independent beyond rounding, from the upper triangle of their Gram matrix, row by row in
+// (real, imaginary) pairs: the pivots of its Cholesky factorisation, each relative to its diagonal
+static bool independent(const double* tri, int nm) {
+  std::vector<double2> L((size_t)nm * nm);   // row j: conj of the Gram matrix's column, then of the factor's
+  for (int i = 0; i < nm; ++i)
+    for (int j = i; j < nm; ++j, tri += 2) L[(size_t)j * nm + i] = make_double2(tri[0], -tri[1]);
+  for (int j = 0; j < nm; ++j) {
+    double2* lj = L.data() + (size_t)j * nm;
+    const double d = lj[j].x;
+    double p = d;
+    for (int k = 0; k < j; ++k) p -= lj[k].x * lj[k].x + lj[k].y * lj[k].y;
+    if (!(p > 1e-12 * d)) return false;   // a zero vector and a NaN, too
+    const double r = 1.0 / std::sqrt(p);
+    for (int i = j + 1; i < nm; ++i) {
+      double2* li = L.data() + (size_t)i * nm;
+      double x = li[j].x, y = li[j].y;
+      for (int k = 0; k < j; ++k) {
+        x -= li[k].x * lj[k].x + li[k].y * lj[k].y;
+        y -= li[k].y * lj[k].x - li[k].x * lj[k].y;
+      }
+      li[j] = make_double2(x * r, y * r);
+    }
+  }
+  return true;
+}
 
 static int tf_setup(bf_handle* h, bf_stack* s, bf_modes* md, int mode, TfCache** out) {
   const bool fp64 = mode == 0;
@@ -2307,25 +2334,32 @@ static int tf_setup(bf_handle* h, bf_stack* s, bf_modes* md, int mode, TfCache**
                                                              c.members.as<int>(), c.tri.as<int2>(), c.K, c.msz,
                                                              (int)npix, scale);
       TCK(cudaGetLastError());
-      TCKS(d_sum.alloc(h, sizeof(double) * 2 * c.T));
+      TCKS(d_sum.alloc(h, sizeof(double) * 4 * c.T));   // of the entries' sizes, then of the entries
+      double* d_sgn = d_sum.as<double>() + 2 * c.T;
       bf::note_launch();
       k_rowsum<double, true><<<2 * c.T, 256, 0, st>>>(d_sum.as<double>(), Ad.as<double>(), c.K);
       TCK(cudaGetLastError());
-      std::vector<double> sum(2 * c.T);
+      bf::note_launch();
+      k_rowsum<<<2 * c.T, 256, 0, st>>>(d_sgn, Ad.as<double>(), c.K);
+      TCK(cudaGetLastError());
+      std::vector<double> sum(4 * c.T);
       TCK(cudaMemcpyAsync(sum.data(), d_sum.p, sizeof(double) * sum.size(), cudaMemcpyDeviceToHost, st));
       TCK(cudaStreamSynchronize(st));
       // A row's product with the phasors is at most its sum of sizes times the largest of them.  The rounding of row
       // (m, m') scales with both modes' transforms, whose sizes the diagonals' real rows give (patterns come in any
       // scale): zero is what four units in the last place of their geometric mean could not show.  Rows that cancel by
       // symmetry sum to 0.2 to 1 of them, the least of the others to 1e14; phasors above 1 (negative distances, gain)
-      // would multiply the rounding that is left out, too.
+      // would multiply the rounding that is left out, too.  Modes that depend on one another (more of them than
+      // pixels) keep every row: without that rounding their matrices can be singular to the bit.
+      c.dependent = !independent(sum.data() + 2 * c.T, nm);
       std::vector<double> diag(nm);
       for (int t = 0, m = 0; m < nm; t += nm - m++) diag[m] = sum[2 * t];
       std::vector<int> rows, map(2 * c.T, -1);
       for (int t = 0, m = 0; m < nm; ++m)
         for (int mp = m; mp < nm; ++mp, ++t)
           for (int r = 2 * t; r < 2 * t + 2; ++r)
-            if (!(sum[r] <= 4 * DBL_EPSILON * std::sqrt(diag[m]) * std::sqrt(diag[mp])) || (m == mp && r == 2 * t)) {
+            if (c.dependent || (m == mp && r == 2 * t) ||
+                !(sum[r] <= 4 * DBL_EPSILON * std::sqrt(diag[m]) * std::sqrt(diag[mp]))) {
               map[r] = (int)rows.size();
               rows.push_back(r);
             }
@@ -2352,14 +2386,9 @@ static int tf_setup(bf_handle* h, bf_stack* s, bf_modes* md, int mode, TfCache**
         k_take_rows_tc<<<dim3(blocks_for(c.Kp), c.Rw), 256, 0, st>>>(c.Wh.as<float>(), c.Wl.as<float>(),
                                                                     Ad.as<double>(), d_rows.as<int>(), c.K, c.Kp);
         TCK(cudaGetLastError());
-        DBuf g;   // of all rows, then of those kept
-        TCKS(g.alloc(h, sizeof(double) * 2 * c.T));
         TCKS(c.gW.alloc(h, sizeof(double) * c.Rw));
         bf::note_launch();
-        k_rowsum<<<2 * c.T, 256, 0, st>>>(g.as<double>(), Ad.as<double>(), c.K);
-        TCK(cudaGetLastError());
-        bf::note_launch();
-        k_take_rows<<<dim3(1, c.Rw), 32, 0, st>>>(c.gW.as<double>(), g.as<double>(), d_rows.as<int>(), 1);
+        k_take_rows<<<dim3(1, c.Rw), 32, 0, st>>>(c.gW.as<double>(), d_sgn, d_rows.as<int>(), 1);
         std::vector<float> kt2(c.K);
         for (int o = 0; o < c.K; ++o) {
           const double kx = s->kX[c.rep_h[o].x], ky = s->kY[c.rep_h[o].y];
@@ -2444,7 +2473,19 @@ static int tf_setup(bf_handle* h, bf_stack* s, bf_modes* md, int mode, TfCache**
       TCK(cudaGetLastError());
     }
   }
+  std::vector<double2> gram(c.herm_w ? 0 : (size_t)nm * nm);
+  if (!c.herm_w)
+    TCK(cudaMemcpyAsync(gram.data(), c.gram.p, sizeof(double2) * gram.size(), cudaMemcpyDeviceToHost, st));
   TCK(cudaStreamSynchronize(st));
+  if (!c.herm_w) {
+    std::vector<double> tri;
+    for (int m = 0; m < nm; ++m)
+      for (int mp = m; mp < nm; ++mp) {
+        tri.push_back(gram[(size_t)m * nm + mp].x);
+        tri.push_back(gram[(size_t)m * nm + mp].y);
+      }
+    c.dependent = !independent(tri.data(), nm);
+  }
   c.U.release();
   c.Phi.release();
   c.modes_id = md->id;
@@ -2653,7 +2694,8 @@ static int tc_class_gemm(bf_handle* h, const float* Ah, const float* Al, int Mp,
   return BF_OK;
 }
 
-// A disk whose tilt and surface factor is 1 everywhere
+// A disk whose tilt and surface factor is 1 everywhere.  (Modes that depend on one another take the general route
+// there, as they keep every row of the gaps: their matrices are regular by rounding alone.)
 static bool flat_disk(const bf_stack* s, const RegionT& r, int j) {
   return r.klass == 1 && r.tx == 0.0 && r.ty == 0.0 && !(s->d_surf && s->surf_nonzero[j]);
 }
@@ -2680,7 +2722,7 @@ static int tf_propagation_matrices(bf_handle* h, bf_stack* s, bf_modes* md, TfCa
   for (int j = j0; j < nd; ++j) {
     if (regs[j].klass == 0) kreg.push_back(j);
     else if (regs[j].klass == 3) freg.push_back(j);
-    else if (flat_disk(s, regs[j], j)) flat.push_back(j);
+    else if (!c.dependent && flat_disk(s, regs[j], j)) flat.push_back(j);
     else preg.push_back(j);
   }
   int* tc_err = reinterpret_cast<int*>(h->d_scalar + 2);   // set by the tensor-core GEMM on a wait timeout
@@ -3165,6 +3207,7 @@ static int tf_run_t(bf_handle* h, bf_stack* s, bf_modes* md, int nf, const doubl
   constexpr bool fp64 = std::is_same<PT, double2>::value;
   cudaStream_t st = h->stream();
   const int nd = s->nd, nm = md->nm;
+  bool dependent = false;   // TfCache::dependent
   std::vector<cd> eps(s->eps);
   if (mirror_1e30)
     for (auto& e : eps)
@@ -3204,6 +3247,7 @@ static int tf_run_t(bf_handle* h, bf_stack* s, bf_modes* md, int nf, const doubl
   } else if (!P_dev) {
     TfCache* c = nullptr;
     TCKS(tf_setup(h, s, md, mode, &c));
+    dependent = c->dependent;
     const int j0 = only_matrices ? 0 : 1;
     TCKS(tf_propagation_matrices<PT>(h, s, md, *c, regs, j0, nf, fv, prop_kind, P, mode, nreq));
   }
@@ -3290,7 +3334,7 @@ static int tf_run_t(bf_handle* h, bf_stack* s, bf_modes* md, int nf, const doubl
     std::vector<int2> copies;
     for (int j = 1; j < nd; ++j) {
       int same = j;
-      if (!pm && !P_dev && flat_disk(s, regs[j], j))
+      if (!pm && !P_dev && !dependent && flat_disk(s, regs[j], j))
         for (same = 1; same < j && !(flat_disk(s, regs[same], same) && same_disk(regs[same], regs[j]));) ++same;
       if (same == j) first.push_back(j);
       if (same != j || (nreq > 1 && regs[j].klass != 0)) copies.push_back(make_int2(j, same));
