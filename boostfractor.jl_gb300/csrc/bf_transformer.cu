@@ -1699,7 +1699,7 @@ __global__ void __launch_bounds__((NB / 2) * (NB / 4), NB == 64 ? 1 : 4)
 // axion beam's boost, 1 the reflection.  8 lanes a matrix row, 4 rows a warp,
 // P's rows then inverse(P)'s; a region's entries are loaded while the region
 // before is finished.  failed[f] is set when the iteration does not converge.
-constexpr int kRefineThreads = 512, kRefineMax = 12;
+constexpr int kRefineThreads = 512;
 __global__ void __launch_bounds__(kRefineThreads, 2)
     k_refine(const float2* P, const float2* Pinv, const float2* X, const int* scales, const ChainRegionDF* cr, int nd,
              int nm, const double2* emit, const double2* reflect, double2* boost, double2* refl, double* beta2, int* failed) {
@@ -1733,7 +1733,10 @@ __global__ void __launch_bounds__(kRefineThreads, 2)
   };
   float last = 0.f;
   bool ok = false, fell = false;
-  for (int it = 0; it < kRefineMax && !ok; ++it) {
+  // A residual takes longer than half the regions' double-float products at 17 modes and a tenth of it at 64, so fewer
+  // modes are given fewer of them.
+  const int most = 3 + nm / 8;
+  for (int it = 0; it < most && !ok; ++it) {
     // the residual: the vector (reflect or 0, x) through the regions, nd - 1 to 1
     fetch(nd - 1);
     if (tid < nm) {
@@ -1825,7 +1828,7 @@ __global__ void __launch_bounds__(kRefineThreads, 2)
     // falling is the residual's rounding
     const bool falls = it > 0 && dn < 0.1f * last;
     if (seen && (dn == 0.f || (falls ? dn * (dn / last) <= 1e-13f * xn : fell && dn <= 1e-6f * xn))) ok = true;
-    else if (!(dn < INFINITY) || (it > 0 && !(dn < 0.5f * last))) break;   // not contracting
+    else if (!(dn < INFINITY) || (it > 0 && !(dn < (it > 1 ? 0.1f : 0.5f) * last))) break;   // not, or slowly, contracting
     fell = falls;
     last = dn;
     __syncthreads();
@@ -3198,6 +3201,33 @@ static int singular_status(bf_handle* h, const int* sing, int nf, const double* 
 // group_regs (a group solve of nreq requests, see bf_transformer_group): the
 // regions of every request, regs[r nd + j]; the results then cover nreq nf
 // frequencies, request r at r nf + f.
+// How far a plane wave's amplitude grows through the regions behind the first at most, at up to 8 of the frequencies:
+// the larger it is (localised waves between strongly reflecting disks), the worse T22 is conditioned.  Loss left out.
+static double plane_wave_growth(const std::vector<RegionT>& regs, int nd, int nf, const double* freqs) {
+  double most = 0.0;
+  const int count = std::min(nf, 8);
+  for (int q = 0; q < count; ++q) {
+    const double k0 = 2 * M_PI / kC * freqs[count > 1 ? (size_t)q * (nf - 1) / (count - 1) : 0];
+    double xr = 0.0, xi = 0.0, yr = 1.0, yi = 0.0;   // the row (T21, T22)
+    double nr = std::sqrt(cd(regs[1].er, regs[1].ei)).real();
+    for (int j = 2; j < nd; ++j) {
+      const double nl = std::sqrt(cd(regs[j].er, regs[j].ei)).real();
+      const double a = (nr + nl) / (2 * nr), b = (nr - nl) / (2 * nr);
+      const double ur = a * xr + b * yr, ui = a * xi + b * yi, vr = b * xr + a * yr, vi = b * xi + a * yi;
+      const double c = std::cos(k0 * nl * regs[j].dz), d = std::sin(k0 * nl * regs[j].dz);
+      xr = ur * c + ui * d;
+      xi = ui * c - ur * d;
+      yr = vr * c - vi * d;
+      yi = vi * c + vr * d;
+      nr = nl;
+    }
+    const double g = std::sqrt(std::max(xr * xr + xi * xi, yr * yr + yi * yi));
+    if (!(g < INFINITY)) return INFINITY;
+    most = std::max(most, g);
+  }
+  return most;
+}
+
 template <typename PT>
 static int tf_run_t(bf_handle* h, bf_stack* s, bf_modes* md, int nf, const double* freqs, int prop_kind,
                     const double* emit, const double* reflect, const double* pm, int pm_per_freq,
@@ -3500,7 +3530,13 @@ static int tf_run_t(bf_handle* h, bf_stack* s, bf_modes* md, int nf, const doubl
       // before them
       TCKS(Wdf.alloc(h, sizeof(DFc) * (size_t)nf * nm * nm));
     }
-    if (nm > 16 && nm <= 64) {
+    // Refined unless most frequencies would come out too badly conditioned for a complex64 inverse and take the chain in
+    // double-float after all: 256 frequencies of 40 disks of eps 24 (growth 1e8 to 1e9) took 1.3 (64 modes) to 1.5 times
+    // (17 modes) as long with the attempt; 20 disks (growth 1e4 to 1e5) take 0.3 to 0.9 of the time with it, 80 disks of
+    // eps 9.4 (growth 8) 0.3 to 0.9.  At 17 modes it pays up to 4e4, at 64 up to 6e5.
+    const bool refine = nm > 16 && nm <= 64 &&
+                        (pm || plane_wave_growth(regs, nd, nf / nreq, freqs) <= std::pow(10.0, 4.2 + nm / 40.0));
+    if (refine) {
       // T22 in complex64 and its inverse share the buffers of the double-float
       // chain, which runs after them, if at all
       const size_t n22 = sizeof(float2) * (size_t)nf * nm * nm;
