@@ -3201,13 +3201,15 @@ static int singular_status(bf_handle* h, const int* sing, int nf, const double* 
 // group_regs (a group solve of nreq requests, see bf_transformer_group): the
 // regions of every request, regs[r nd + j]; the results then cover nreq nf
 // frequencies, request r at r nf + f.
-// How far a plane wave's amplitude grows through the regions behind the first at most, at up to 8 of the frequencies:
-// the larger it is (localised waves between strongly reflecting disks), the worse T22 is conditioned.  Loss left out.
-static double plane_wave_growth(const std::vector<RegionT>& regs, int nd, int nf, const double* freqs) {
+// How far a plane wave's amplitude grows through the regions behind the first at most, at up to 8 of the frequencies
+// (of a group's requests in turn, each at least once): the larger it is (localised waves between strongly reflecting
+// disks), the worse T22 is conditioned.  Loss left out.
+static double plane_wave_growth(const std::vector<RegionT>& all, int nd, int nf, const double* freqs, int nreq) {
   double most = 0.0;
-  const int count = std::min(nf, 8);
+  const int count = std::max(std::min(nf, 8), nreq);
   for (int q = 0; q < count; ++q) {
     const double k0 = 2 * M_PI / kC * freqs[count > 1 ? (size_t)q * (nf - 1) / (count - 1) : 0];
+    const RegionT* regs = all.data() + (size_t)(q % nreq) * nd;
     double xr = 0.0, xi = 0.0, yr = 1.0, yi = 0.0;   // the row (T21, T22)
     double nr = std::sqrt(cd(regs[1].er, regs[1].ei)).real();
     for (int j = 2; j < nd; ++j) {
@@ -3535,7 +3537,7 @@ static int tf_run_t(bf_handle* h, bf_stack* s, bf_modes* md, int nf, const doubl
     // (17 modes) as long with the attempt; 20 disks (growth 1e4 to 1e5) take 0.3 to 0.9 of the time with it, 80 disks of
     // eps 9.4 (growth 8) 0.3 to 0.9.  At 17 modes it pays up to 4e4, at 64 up to 6e5.
     const bool refine = nm > 16 && nm <= 64 &&
-                        (pm || plane_wave_growth(regs, nd, nf / nreq, freqs) <= std::pow(10.0, 4.2 + nm / 40.0));
+                        (pm || plane_wave_growth(regs, nd, nf / nreq, freqs, nreq) <= std::pow(10.0, 4.2 + nm / 40.0));
     if (refine) {
       // T22 in complex64 and its inverse share the buffers of the double-float
       // chain, which runs after them, if at all
